@@ -1354,7 +1354,9 @@ int evaluate_both_dev(wdl_ctx* ctx, int P, int K, int L, int loss_type, double s
   if ((size_t)n != PK + KN) return set_error(ctx, WDL_ERR_INVALID_ARG, "n != P*K + K*N");
   // Staging: v2 weights [PK], v2 atoms [KN], la [PK], dic [KN], loss [P].
   const size_t stage = 8 * (2 * PK + 2 * KN + P) + 5 * 256;
-  const size_t main = eval_bytes(ctx, P, K, L);
+  // The workspace's size may be odd (it can end in sign bytes or an odd number of
+  // floats): the doubles of the staging start on the next 256 bytes.
+  const size_t main = (eval_bytes(ctx, P, K, L) + 255) & ~size_t(255);
   int rc;
   if ((rc = ensure_arena(ctx, main + stage))) return rc;
   char* tail = static_cast<char*>(ctx->arena.ptr) + main;
