@@ -450,6 +450,13 @@ int conv_stack_simt(wdl_ctx* ctx, const T* in, T* out, T* tmp, size_t nimg, cuda
   const size_t N = ctx->N;
   ConvTimer timer(ctx, s, nimg);
   int rc;
+  if (band_fits<T>(ctx, 0)) {
+    rc = ctx->ndim == 2 ? band_conv<T, T, T>(ctx, in, out, tmp, nullptr, nimg, s)
+                        : band_conv<T, T, T>(ctx, in, out, out, tmp, nimg, s);
+    if (rc) return rc;
+    timer.done();
+    return WDL_OK;
+  }
   if (ctx->ndim == 2) {
     if ((rc = axis_pass<T>(ctx, in, tmp, factor<T>(ctx, 0), H, W, nimg, N, s))) return rc;
     if ((rc = axis_pass<T>(ctx, tmp, out, factor<T>(ctx, 1), W, H, nimg, N, s))) return rc;

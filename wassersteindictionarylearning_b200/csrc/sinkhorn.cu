@@ -23,87 +23,6 @@
 namespace wdl {
 namespace {
 
-template <typename T>
-__device__ __forceinline__ T d_exp(T x);
-template <>
-__device__ __forceinline__ float d_exp<float>(float x) { return expf(x); }
-template <>
-__device__ __forceinline__ double d_exp<double>(double x) { return exp(x); }
-template <typename T>
-__device__ __forceinline__ T d_log(T x);
-template <>
-__device__ __forceinline__ float d_log<float>(float x) { return logf(x); }
-template <>
-__device__ __forceinline__ double d_log<double>(double x) { return log(x); }
-// Natural log of a magnitude feeding a log-domain operand: FP32 takes the
-// hardware base-2 logarithm times ln 2 (absolute error ~2e-7, i.e. ~2e-7
-// relative on the scaling it encodes; a log-domain value of magnitude >= 2 is
-// rounded more coarsely than that anyway); FP64 the library log.
-template <typename T>
-__device__ __forceinline__ T d_log_mag(T x);
-template <>
-__device__ __forceinline__ float d_log_mag<float>(float x) {
-  float y;
-  asm("lg2.approx.f32 %0, %1;" : "=f"(y) : "f"(fabsf(x)));
-  return y * 0.6931471805599453f;
-}
-template <>
-__device__ __forceinline__ double d_log_mag<double>(double x) { return log(fabs(x)); }
-
-// safe_log = log(max(EPSILON, x)) (cpp/loss.h:3-5).
-template <typename T>
-__device__ __forceinline__ T safe_log(T x);
-template <>
-__device__ __forceinline__ double safe_log<double>(double x) {
-  return log(x > kEpsilon ? x : kEpsilon);
-}
-template <>
-__device__ __forceinline__ float safe_log<float>(float x) {
-  return x > 0.f ? logf(x) : float(kLogEpsilon);
-}
-
-// Logarithms that are summed in FP64 (grid reductions, the geometric mean over
-// atoms): FP64 mode uses log directly; FP32 mode uses the split form of
-// log_f32_precise so the FP64 sum is not limited by logf's absolute error.
-template <typename T>
-__device__ __forceinline__ double acc_log(T x);
-template <>
-__device__ __forceinline__ double acc_log<double>(double x) { return log(x); }
-template <>
-__device__ __forceinline__ double acc_log<float>(float x) {
-  return x > 0.f ? log_f32_precise(x) : (double)logf(x);
-}
-template <typename T>
-__device__ __forceinline__ double acc_safe_log(T x);
-template <>
-__device__ __forceinline__ double acc_safe_log<double>(double x) {
-  return log(x > kEpsilon ? x : kEpsilon);
-}
-template <>
-__device__ __forceinline__ double acc_safe_log<float>(float x) {
-  return x > 0.f ? log_f32_precise(x) : kLogEpsilon;
-}
-template <typename T>
-__device__ __forceinline__ T exp_from(double s);
-template <>
-__device__ __forceinline__ double exp_from<double>(double s) { return exp(s); }
-template <>
-__device__ __forceinline__ float exp_from<float>(double s) { return exp_to_f32(s); }
-
-__device__ __forceinline__ double block_sum(double v, double* sh) {
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  const int w = threadIdx.x >> 5, l = threadIdx.x & 31, nw = blockDim.x >> 5;
-  __syncthreads();
-  if (l == 0) sh[w] = v;
-  __syncthreads();
-  double t = 0;
-  if (threadIdx.x < 32) {
-    t = threadIdx.x < nw ? sh[threadIdx.x] : 0.0;
-    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-  }
-  return t;  // valid in thread 0
-}
-
 #define GRID_STRIDE(i, n) \
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < (n); i += (size_t)gridDim.x * blockDim.x)
 
@@ -782,8 +701,8 @@ int launch_cfg(wdl_ctx* ctx, size_t n) { return grid_for(n, 256, ctx->sm_count, 
 
 // Nested Sinkhorn of the Wasserstein loss (cpp/loss.h:92-154) on all P
 // barycenters at once, kernel domain, 50 inner iterations.
-template <typename T>
-int wasserstein_loss(wdl_ctx* ctx, EvalBufs<T>& B, const double* obs, int P, cudaStream_t s) {
+template <typename T, class Bufs>
+int wasserstein_loss(wdl_ctx* ctx, Bufs& B, const T* bary, const double* obs, int P, cudaStream_t s) {
   const size_t N = ctx->N, PN = (size_t)P * N;
   const unsigned G = launch_cfg(ctx, PN);
   int rc;
@@ -791,14 +710,14 @@ int wasserstein_loss(wdl_ctx* ctx, EvalBufs<T>& B, const double* obs, int P, cud
   WDL_LAUNCH_CHECK(ctx);
   for (int it = 0; it < 50; ++it) {
     if ((rc = conv_stack<T>(ctx, B.wb, B.wc, B.ctmp, P, s))) return rc;
-    k_ratio<T><<<G, 256, 0, s>>>(B.bary, nullptr, B.wc, B.wa, PN);
+    k_ratio<T><<<G, 256, 0, s>>>(bary, nullptr, B.wc, B.wa, PN);
     WDL_LAUNCH_CHECK(ctx);
     if ((rc = conv_stack<T>(ctx, B.wa, B.wc, B.ctmp, P, s))) return rc;
     k_ratio<T><<<G, 256, 0, s>>>(nullptr, obs, B.wc, B.wb, PN);
     WDL_LAUNCH_CHECK(ctx);
   }
   if ((rc = conv_stack<T>(ctx, B.wb, B.wc, B.ctmp, P, s))) return rc;
-  k_wloss<T><<<P, 256, 0, s>>>(B.bary, obs, B.wa, B.wb, B.wc, B.wgrad, B.loss, ctx->gamma, N);
+  k_wloss<T><<<P, 256, 0, s>>>(bary, obs, B.wa, B.wb, B.wc, B.wgrad, B.loss, ctx->gamma, N);
   WDL_LAUNCH_CHECK(ctx);
   return WDL_OK;
 }
@@ -878,7 +797,7 @@ int gradient_both_t(wdl_ctx* ctx, int P, int K, int L, int loss_type, const doub
   }
 
   // Loss and its gradient (:597).
-  if (wloss && (rc = wasserstein_loss<T>(ctx, B, observed, P, s))) return rc;
+  if (wloss && (rc = wasserstein_loss<T>(ctx, B, B.bary, observed, P, s))) return rc;
   k_loss<T><<<P, 256, 0, s>>>(B.bary, observed, B.wgrad, B.n, B.gw, B.loss, loss_type, N);
   WDL_LAUNCH_CHECK(ctx);
 
@@ -1047,6 +966,174 @@ int barycenter_t(wdl_ctx* ctx, int P, int K, int L, const double* atoms, const d
     WDL_LAUNCH_CHECK(ctx);
   }
   k_cast_back<T><<<launch_cfg(ctx, PN), 256, 0, s>>>(bary, bary_out, PN);
+  WDL_LAUNCH_CHECK(ctx);
+  return WDL_OK;
+}
+
+// The CUDA-core kernel domain with whole lines in shared memory
+// (sinkhorn_band.cu): two launches per iteration and per reverse round.
+template <typename T>
+struct BandBufs {
+  double *atoms64, *lam64;
+  T *atoms, *lam, *b0 = nullptr;
+  BandEval<T> e{};
+  T *wa = nullptr, *wb = nullptr, *wc = nullptr, *wgrad = nullptr, *ctmp = nullptr;
+  double* loss = nullptr;
+  template <class A>
+  void layout(A& al, const wdl_ctx* ctx, size_t P, size_t K, size_t L, bool b_init, bool fwd_only, bool wloss) {
+    const size_t N = ctx->N, KN = K * N, PKN = P * KN, PN = P * N;
+    auto t = [&](T*& p, size_t n) { alloc_into(al, reinterpret_cast<void**>(&p), n * sizeof(T)); };
+    auto d = [&](double*& p, size_t n) { alloc_into(al, reinterpret_cast<void**>(&p), n * 8); };
+    d(atoms64, KN);
+    d(lam64, P * K);
+    t(atoms, KN);
+    t(lam, P * K);
+    if (b_init) t(b0, PKN);
+    alloc_into(al, reinterpret_cast<void**>(&e.range), P * sizeof(int));
+    t(e.bary, fwd_only ? PN : L * PN);
+    t(e.t1, fwd_only ? PKN : 2 * PKN);
+    t(e.t2, fwd_only ? PKN : 2 * PKN);
+    if (!fwd_only) {
+      t(e.cb, L * PKN);
+      t(e.phi, L * PKN);
+      t(e.q, PKN);
+      t(e.n, PN);
+      t(e.gw, PN);
+      d(e.gdic, KN);
+      d(e.dotp, P * K * band_dot_parts<T>(ctx, (int)K));
+      d(e.dot, P * K);
+      d(e.lossp, P * band_loss_parts(ctx));
+      d(loss, P);
+    }
+    if (wloss) {
+      t(wa, PN);
+      t(wb, PN);
+      t(wc, PN);
+      t(wgrad, PN);
+      t(ctmp, PN);
+    }
+    e.P = (int)P;
+    e.K = (int)K;
+    e.L = (int)L;
+    e.atoms = atoms;
+    e.lam = lam;
+    e.lam64 = lam64;
+  }
+};
+
+template <typename T>
+size_t band_bytes(const wdl_ctx* ctx, size_t P, size_t K, size_t L, bool b_init, bool fwd_only, bool wloss) {
+  ArenaPlan plan;
+  BandBufs<T> b;
+  b.layout(plan, ctx, P, K, L, b_init, fwd_only, wloss);
+  return plan.off + 256;
+}
+
+// Kernel-domain contexts without tensor cores whose lines fit.
+bool use_band(const wdl_ctx* ctx, int K) {
+  if (ctx->domain != WDL_DOMAIN_KERNEL || ctx->tc) return false;
+  return ctx->precision == WDL_FP64 ? band_fits<double>(ctx, K) : band_fits<float>(ctx, K);
+}
+
+// Inputs: normalised FP64 copies (normalize_values, :562) and their T casts.
+template <typename T>
+int band_inputs(wdl_ctx* ctx, BandBufs<T>& B, int P, int K, const double* atoms, const double* weights,
+                bool normalise, cudaStream_t s) {
+  const size_t N = ctx->N, KN = (size_t)K * N;
+  if (normalise) {
+    k_normalise_rows<<<K, 256, 0, s>>>(atoms, B.atoms64, N, 0.0);
+    WDL_LAUNCH_CHECK(ctx);
+    k_normalise_rows<<<P, 32, 0, s>>>(weights, B.lam64, K, 0.0);
+    WDL_LAUNCH_CHECK(ctx);
+  } else {
+    WDL_CUDA_TRY(ctx, cudaMemcpyAsync(B.atoms64, atoms, KN * 8, cudaMemcpyDeviceToDevice, s));
+    WDL_CUDA_TRY(ctx, cudaMemcpyAsync(B.lam64, weights, (size_t)P * K * 8, cudaMemcpyDeviceToDevice, s));
+  }
+  k_cast<T><<<launch_cfg(ctx, KN), 256, 0, s>>>(B.atoms64, B.atoms, KN);
+  WDL_LAUNCH_CHECK(ctx);
+  k_cast<T><<<1, 256, 0, s>>>(B.lam64, B.lam, (size_t)P * K);
+  WDL_LAUNCH_CHECK(ctx);
+  if (sizeof(T) == 4) {
+    WDL_CUDA_TRY(ctx, cudaMemsetAsync(B.e.range, 0, (size_t)P * sizeof(int), s));
+  } else {
+    B.e.range = nullptr;
+  }
+  return WDL_OK;
+}
+
+// b[L] = bary[L] / phi[L] (the warm-restart store).
+template <typename T>
+__global__ void k_band_b_last(const T* __restrict__ bary, const T* __restrict__ phi, double* __restrict__ out,
+                              int K, size_t N, size_t PKN) {
+  GRID_STRIDE(i, PKN) {
+    const size_t p = i / ((size_t)K * N), j = i % N;
+    out[i] = (double)(bary[p * N + j] / phi[i]);
+  }
+}
+
+template <typename T>
+int gradient_band_t(wdl_ctx* ctx, int P, int K, int L, int loss_type, const double* atoms,
+                    const double* weights, const double* observed, const double* b_init,
+                    double* result_la, double* result_dic, double* bary_out, double* loss_out,
+                    double* b_last, cudaStream_t s, bool normalise) {
+  const bool wloss = loss_type == WDL_LOSS_WASSERSTEIN;
+  const size_t N = ctx->N, KN = (size_t)K * N, PKN = (size_t)P * KN, PN = (size_t)P * N;
+  int rc;
+  if ((rc = ensure_arena(ctx, band_bytes<T>(ctx, P, K, L, b_init != nullptr, false, wloss)))) return rc;
+  ctx->arena.reset();
+  BandBufs<T> B;
+  B.layout(ctx->arena, ctx, P, K, L, b_init != nullptr, false, wloss);
+  if ((rc = band_inputs(ctx, B, P, K, atoms, weights, normalise, s))) return rc;
+  if (b_init) {
+    k_cast<T><<<launch_cfg(ctx, PKN), 256, 0, s>>>(b_init, B.b0, PKN);
+    WDL_LAUNCH_CHECK(ctx);
+  }
+  BandEval<T>& e = B.e;
+  e.dict = result_dic ? 1 : 0;
+  if ((rc = band_forward<T>(ctx, e, B.b0, s))) return rc;
+  T* bary = e.bary + (size_t)(L - 1) * PN;
+  const unsigned G_PN = launch_cfg(ctx, PN);
+  if (e.range) {
+    k_poison_out_of_range<T><<<G_PN, 256, 0, s>>>(bary, e.range, N, PN);
+    WDL_LAUNCH_CHECK(ctx);
+  }
+  if (wloss && (rc = wasserstein_loss<T>(ctx, B, bary, observed, P, s))) return rc;
+  if ((rc = band_loss<T>(ctx, e, observed, B.wgrad, loss_type, s))) return rc;
+  WDL_CUDA_TRY(ctx, cudaMemsetAsync(e.dotp, 0, (size_t)P * K * band_dot_parts<T>(ctx, (int)K) * sizeof(double), s));
+  if (e.dict) WDL_CUDA_TRY(ctx, cudaMemsetAsync(e.gdic, 0, KN * sizeof(double), s));
+  if ((rc = band_backward<T>(ctx, e, wloss ? nullptr : B.loss, s))) return rc;
+
+  WDL_CUDA_TRY(ctx, cudaMemcpyAsync(result_la, e.dot, (size_t)P * K * 8, cudaMemcpyDeviceToDevice, s));
+  if (result_dic)
+    WDL_CUDA_TRY(ctx, cudaMemcpyAsync(result_dic, e.gdic, KN * sizeof(double), cudaMemcpyDeviceToDevice, s));
+  if (bary_out) {
+    k_cast_back<T><<<G_PN, 256, 0, s>>>(bary, bary_out, PN);
+    WDL_LAUNCH_CHECK(ctx);
+  }
+  if (loss_out) WDL_CUDA_TRY(ctx, cudaMemcpyAsync(loss_out, B.loss, (size_t)P * 8, cudaMemcpyDeviceToDevice, s));
+  if (b_last) {
+    k_band_b_last<T><<<launch_cfg(ctx, PKN), 256, 0, s>>>(bary, e.phi + (size_t)(L - 1) * PKN, b_last, K, N, PKN);
+    WDL_LAUNCH_CHECK(ctx);
+  }
+  return WDL_OK;
+}
+
+template <typename T>
+int barycenter_band_t(wdl_ctx* ctx, int P, int K, int L, const double* atoms, const double* weights,
+                      double* bary_out, cudaStream_t s) {
+  const size_t N = ctx->N, PN = (size_t)P * N;
+  int rc;
+  if ((rc = ensure_arena(ctx, band_bytes<T>(ctx, P, K, L, false, true, false)))) return rc;
+  ctx->arena.reset();
+  BandBufs<T> B;
+  B.layout(ctx->arena, ctx, P, K, L, false, true, false);
+  if ((rc = band_inputs(ctx, B, P, K, atoms, weights, true, s))) return rc;
+  if ((rc = band_forward<T>(ctx, B.e, nullptr, s))) return rc;
+  if (B.e.range) {
+    k_poison_out_of_range<T><<<launch_cfg(ctx, PN), 256, 0, s>>>(B.e.bary, B.e.range, N, PN);
+    WDL_LAUNCH_CHECK(ctx);
+  }
+  k_cast_back<T><<<launch_cfg(ctx, PN), 256, 0, s>>>(B.e.bary, bary_out, PN);
   WDL_LAUNCH_CHECK(ctx);
   return WDL_OK;
 }
@@ -1226,12 +1313,18 @@ size_t eval_bytes(const wdl_ctx* ctx, int P, int K, int L) {
     const size_t b = eval_bytes_t<float>(P, K, L, ctx->N, false, true);  // Wasserstein loss runs unfused
     return a > b ? a : b;
   }
+  if (use_band(ctx, K))
+    return use_fp64(ctx) ? band_bytes<double>(ctx, P, K, L, true, false, true)
+                         : band_bytes<float>(ctx, P, K, L, true, false, true);
   return use_fp64(ctx) ? eval_bytes_t<double>(P, K, L, ctx->N, log_domain, true)
                        : eval_bytes_t<float>(P, K, L, ctx->N, log_domain, true);
 }
 
 size_t barycenter_bytes(const wdl_ctx* ctx, int P, int K) {
   if (tc_fused(ctx) && ctx->domain == WDL_DOMAIN_KERNEL) return fused_bytes(P, K, 2, ctx->N, false, true);
+  if (use_band(ctx, K))
+    return use_fp64(ctx) ? band_bytes<double>(ctx, P, K, 1, false, true, false)
+                         : band_bytes<float>(ctx, P, K, 1, false, true, false);
   const size_t N = ctx->N, KN = (size_t)K * N, PKN = (size_t)P * KN, PN = (size_t)P * N;
   const size_t t = use_fp64(ctx) ? 8 : 4;
   return 8 * (KN + (size_t)P * K) + t * (KN + (size_t)P * K + 4 * PKN + PN) + 4 * (size_t)P + 17 * 256;
@@ -1303,9 +1396,12 @@ int gradient_both_dev(wdl_ctx* ctx, int P, int K, int L, int loss_type, const do
   // the workspace is sized before the key is formed, so a replay never needs
   // a larger one
   const bool f64 = use_fp64(ctx);
-  const bool log_domain = ctx->domain == WDL_DOMAIN_LOG;
-  const size_t need = f64 ? eval_bytes_t<double>(P, K, L, ctx->N, log_domain, loss_type == WDL_LOSS_WASSERSTEIN)
-                          : eval_bytes_t<float>(P, K, L, ctx->N, log_domain, loss_type == WDL_LOSS_WASSERSTEIN);
+  const bool log_domain = ctx->domain == WDL_DOMAIN_LOG, wloss = loss_type == WDL_LOSS_WASSERSTEIN;
+  const bool band = use_band(ctx, K);
+  const size_t need = band ? (f64 ? band_bytes<double>(ctx, P, K, L, b_init != nullptr, false, wloss)
+                                  : band_bytes<float>(ctx, P, K, L, b_init != nullptr, false, wloss))
+                      : f64 ? eval_bytes_t<double>(P, K, L, ctx->N, log_domain, wloss)
+                            : eval_bytes_t<float>(P, K, L, ctx->N, log_domain, wloss);
   int rc;
   if ((rc = ensure_arena(ctx, need))) return rc;
   const unsigned long long key[20] = {
@@ -1318,6 +1414,11 @@ int gradient_both_dev(wdl_ctx* ctx, int P, int K, int L, int loss_type, const do
       (unsigned long long)(uintptr_t)b_last, (unsigned long long)(uintptr_t)s,
       (unsigned long long)(uintptr_t)ctx->arena.ptr, (unsigned long long)ctx->arena.bytes, 0ull, 0ull};
   return replay_or_run(ctx, key, s, [&]() {
+    if (band)
+      return f64 ? gradient_band_t<double>(ctx, P, K, L, loss_type, atoms, weights, observed, b_init, result_la,
+                                           result_dic, bary, loss, b_last, s, normalise)
+                 : gradient_band_t<float>(ctx, P, K, L, loss_type, atoms, weights, observed, b_init, result_la,
+                                          result_dic, bary, loss, b_last, s, normalise);
     if (f64)
       return gradient_both_t<double>(ctx, P, K, L, loss_type, atoms, weights, observed, b_init,
                                      result_la, result_dic, bary, loss, b_last, s, normalise);
@@ -1339,6 +1440,9 @@ int barycenter_dev(wdl_ctx* ctx, int P, int K, int L, const double* atoms, const
       (unsigned long long)(uintptr_t)bary, 0ull, 0ull, 0ull, 0ull, (unsigned long long)(uintptr_t)s,
       (unsigned long long)(uintptr_t)ctx->arena.ptr, (unsigned long long)ctx->arena.bytes, 0ull, 0ull};
   return replay_or_run(ctx, key, s, [&]() {
+    if (use_band(ctx, K))
+      return use_fp64(ctx) ? barycenter_band_t<double>(ctx, P, K, L, atoms, weights, bary, s)
+                           : barycenter_band_t<float>(ctx, P, K, L, atoms, weights, bary, s);
     if (use_fp64(ctx)) return barycenter_t<double>(ctx, P, K, L, atoms, weights, bary, s);
     return barycenter_t<float>(ctx, P, K, L, atoms, weights, bary, s);
   });

@@ -209,6 +209,39 @@ inline int log_conv_stack<double>(wdl_ctx* ctx, const double* in, double* out, d
   return log_conv_stack_f64(ctx, in, out, tmp, nimg, is, os, ts, s, sf, so, sp);
 }
 
+// ---- banded CUDA-core forms (sinkhorn_band.cu) ---------------------------------------
+// One kernel-domain evaluation's device buffers: atoms [K][N], lam [P][K] in T
+// and FP64, the iterate store (conv_b, phi [L][P][K][N] and bary [L][P][N]; a
+// barycenter-only run has no conv_b, no phi and one bary), transposed images t1
+// and t2 ([dictionary | weights][P][K][N]; barycenters one [P][K][N]), c / conv_b
+// of a round q [P][K][N], the loss gradient n and n * bary gw [P][N], the atom
+// gradient gdic [K][N], partial dot products and losses (band_dot_parts per
+// (p, k), band_loss_parts per p), dot [P][K], range [P] (FP32) or null.
+template <typename T>
+struct BandEval {
+  int P, K, L, dict;
+  const T *atoms, *lam;
+  const double* lam64;
+  T *cb, *phi, *bary, *t1, *t2, *q, *n, *gw;
+  double *gdic, *dotp, *dot, *lossp;
+  int* range;
+};
+// Whether the lines of a call fit shared memory (K = 0: the operator alone).
+template <typename T>
+bool band_fits(const wdl_ctx* ctx, int K);
+template <typename T>
+size_t band_dot_parts(const wdl_ctx* ctx, int K);
+size_t band_loss_parts(const wdl_ctx* ctx);
+template <typename TI, typename T, typename TO>
+int band_conv(wdl_ctx* ctx, const TI* in, TO* out, T* tmp, T* tmp2, size_t nimg, cudaStream_t s);
+template <typename T>
+int band_forward(wdl_ctx* ctx, const BandEval<T>& e, const T* b0, cudaStream_t s);
+template <typename T>
+int band_loss(wdl_ctx* ctx, const BandEval<T>& e, const double* obs, const T* wgrad, int loss_type,
+              cudaStream_t s);
+template <typename T>
+int band_backward(wdl_ctx* ctx, const BandEval<T>& e, double* loss, cudaStream_t s);
+
 // Tensor-core resources (conv_tc.cu).
 int tc_init(wdl_ctx* ctx);
 void tc_free(wdl_ctx* ctx);
