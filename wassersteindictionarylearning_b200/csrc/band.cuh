@@ -258,9 +258,13 @@ __device__ __forceinline__ void dense8(const typename Vec<T>::V* line, const Axi
     }
 }
 
-// q = i / n for 0 <= i < 65536, with inv from div_magic(n).
-__device__ __forceinline__ uint32_t div_magic(int n) { return n > 1 ? 0xffffffffu / (uint32_t)n + 1u : 0u; }
-__device__ __forceinline__ int fast_div(int i, int n, uint32_t inv) { return n > 1 ? (int)__umulhi((uint32_t)i, inv) : i; }
+// Division of 0 <= i < 65536 by a number that the host knows.
+struct Div {
+  int n;
+  uint32_t inv;
+  __host__ static Div by(int n) { return {n, n > 1 ? 0xffffffffu / (uint32_t)n + 1u : 0u}; }
+  __device__ __forceinline__ int operator()(int i) const { return n > 1 ? (int)__umulhi((uint32_t)i, inv) : i; }
+};
 
 // Items of one pass: the eight-output groups of nl lines, lanes over the lines
 // first; warp w of nw takes items 32 w .. 32 w + 31, and so on.  pre(line, c0,
@@ -269,15 +273,15 @@ __device__ __forceinline__ int fast_div(int i, int n, uint32_t inv) { return n >
 // dropped).  xmag bounds the lines.
 template <typename T, int NE, class Pre, class Sink>
 __device__ __forceinline__ void fir_lines(const typename Vec<T>::V* lines, const typename Vec<T>::V* g,
-                                          const Axis<T>& ax, int nl, uint32_t inv, int xmag, int warp, int nw,
-                                          int lane, Pre pre, Sink sink) {
+                                          const Axis<T>& ax, Div nl, int xmag, int warp, int nw, int lane, Pre pre,
+                                          Sink sink) {
   using V = typename Vec<T>::V;
   constexpr int W = Vec<T>::W;
-  const int items = nl * ax.G;
+  const int items = nl.n * ax.G;
   for (int i0 = warp * 32; i0 < items; i0 += nw * 32) {
     const int it = i0 + lane;
     const bool ok = it < items;
-    const int grp = ok ? fast_div(it, nl, inv) : 0, line = ok ? it - grp * nl : 0;
+    const int grp = ok ? nl(it) : 0, line = ok ? it - grp * nl.n : 0;
     const int c0 = grp * 8;
     const V* lp = lines + line * ax.pitch;
     T ext[NE > 0 ? NE : 1][8][W];

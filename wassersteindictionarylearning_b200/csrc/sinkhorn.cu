@@ -13,6 +13,8 @@
 // one kernel per round; every reduction over the grid or the batch (loss,
 // weight-gradient dot products, the sum of the dictionary gradient over P) runs
 // in FP64.
+#include <cooperative_groups.h>
+
 #include <cmath>
 #include <cstring>
 #include <functional>
@@ -43,25 +45,55 @@ __global__ void k_log_of(const double* __restrict__ in, T* __restrict__ out, siz
   GRID_STRIDE(i, n) out[i] = (T)log(in[i]);
 }
 
-// Problem::normalize_values (cpp/inverseWasserstein.h:53-74), one row per block.
-// With exp_scale != 0 the row is first mapped through exp(v / exp_scale)
-// (evaluate_both's return to the original domain, :997-1011).
-__global__ void k_normalise_rows(const double* __restrict__ in, double* __restrict__ out,
-                                 size_t len, double exp_scale) {
-  __shared__ double sh[32];
-  const double* r = in + (size_t)blockIdx.x * len;
-  double* o = out + (size_t)blockIdx.x * len;
+// Sum over the blocks of a cluster, in rank order (every thread of the cluster
+// calls this; every thread gets the sum).  A row of an image is long enough to
+// keep one SM busy for 40-200 us (100 us at 272 x 240, 190 us at 48^3, mostly load
+// latency), so rows of kRowSplit values or more are shared by a cluster of
+// kRowBlocks blocks: 98 -> 9 us and 190 -> 14 us.  Weight rows keep one warp.
+constexpr int kRowBlocks = 8;
+constexpr size_t kRowSplit = 2048;
+__device__ __forceinline__ double cluster_sum(double v, double* sh) {
+  namespace cg = cooperative_groups;
+  cg::cluster_group c = cg::this_cluster();
+  v = block_sum(v, sh);
+  if (threadIdx.x == 0) sh[32] = v;
+  c.sync();
+  double t = 0;
+  for (unsigned r = 0; r < c.num_blocks(); ++r) t += *c.map_shared_rank(sh + 32, r);
+  c.sync();  // nobody leaves (or reuses sh) while its sum is read
+  return t;
+}
+
+// Problem::normalize_values (cpp/inverseWasserstein.h:53-74), one row per
+// cluster.  With exp_scale != 0 the row is first mapped through
+// exp(v / exp_scale) (evaluate_both's return to the original domain,
+// :997-1011).  cast, when given, receives the values in T (their logarithms
+// when logs is set).
+template <typename T>
+__global__ void __launch_bounds__(512) k_normalise_rows(const double* __restrict__ in, double* __restrict__ out,
+                                                        size_t len, double exp_scale, T* __restrict__ cast,
+                                                        int logs) {
+  __shared__ double sh[33];
+  namespace cg = cooperative_groups;
+  const cg::cluster_group c = cg::this_cluster();
+  const size_t nb = c.num_blocks(), row = blockIdx.x / nb;
+  const size_t step = nb * blockDim.x, first = c.block_rank() * (size_t)blockDim.x + threadIdx.x;
+  const double* r = in + row * len;
+  double* o = out + row * len;
   double s = 0;
-  for (size_t j = threadIdx.x; j < len; j += blockDim.x) {
-    double v = exp_scale != 0.0 ? exp(r[j] / exp_scale) : r[j];
+#pragma unroll 4
+  for (size_t j = first; j < len; j += step) {
+    const double v = exp_scale != 0.0 ? exp(r[j] / exp_scale) : r[j];
     o[j] = v;
     s += v;
   }
-  s = block_sum(s, sh);
-  if (threadIdx.x == 0) sh[0] = s;
-  __syncthreads();
-  s = sh[0];
-  for (size_t j = threadIdx.x; j < len; j += blockDim.x) o[j] = o[j] / s;
+  s = cluster_sum(s, sh);
+#pragma unroll 4
+  for (size_t j = first; j < len; j += step) {
+    const double v = o[j] / s;
+    o[j] = v;
+    if (cast) cast[row * len + j] = logs ? (T)log(v) : (T)v;
+  }
 }
 
 // ---------------- kernel-domain forward (cpp/inverseWasserstein.h:565-593) -----------
@@ -139,43 +171,12 @@ __global__ void k_exp_inplace(T* __restrict__ v, size_t n) {
   GRID_STRIDE(i, n) v[i] = d_exp<T>(v[i]);
 }
 
-// ---------------- loss (cpp/loss.h:19-90), one histogram per block ------------------
-// Writes the loss gradient g into n (the dictionary recursion's start) and
-// g * bary into gw (the weight recursion's start, :633-635).
-template <typename T>
-__global__ void k_loss(const T* __restrict__ bary, const double* __restrict__ obs,
-                       const T* __restrict__ wgrad, T* __restrict__ n, T* __restrict__ gw,
-                       double* __restrict__ loss, int loss_type, size_t N) {
-  __shared__ double sh[32];
-  const size_t p = blockIdx.x;
-  double acc = 0;
-  for (size_t j = threadIdx.x; j < N; j += blockDim.x) {
-    const size_t i = p * N + j;
-    const T v1 = bary[i];
-    const double o = obs[i];
-    const T v2 = (T)o;
-    T g;
-    if (loss_type == WDL_LOSS_TV) {
-      const T d = v1 - v2;
-      acc += fabs((double)v1 - o);
-      g = d > T(0) ? T(0.5) : T(-0.5);
-    } else if (loss_type == WDL_LOSS_QUADRATIC) {
-      const double d = (double)v1 - o;
-      acc += d * d;
-      g = T(2) * (v1 - v2);
-    } else if (loss_type == WDL_LOSS_KL) {
-      const double r = (double)v1 / o;
-      acc += (double)v1 * log(r > kEpsilon ? r : kEpsilon) - (double)v1 + o;
-      g = safe_log<T>(v1 / v2);
-    } else {  // Wasserstein: gradient precomputed by the nested Sinkhorn
-      g = wgrad[i];
-    }
-    n[i] = g;
-    gw[i] = g * v1;
-  }
-  acc = block_sum(acc, sh);
-  if (threadIdx.x == 0 && loss_type != WDL_LOSS_WASSERSTEIN)
-    loss[p] = loss_type == WDL_LOSS_TV ? 0.5 * acc : acc;
+// One histogram's loss from its segments, a warp each.
+__global__ void k_add_segments(const double* __restrict__ part, double* __restrict__ loss, int nseg) {
+  double s = 0;
+  for (int i = threadIdx.x; i < nseg; i += 32) s += part[(size_t)blockIdx.x * nseg + i];
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if (threadIdx.x == 0) loss[blockIdx.x] = s;
 }
 
 // Wasserstein loss helpers (cpp/loss.h:92-154): a = v1 / Kb, b = v2 / Ka.
@@ -586,19 +587,21 @@ __global__ void k_project_weights(const double* __restrict__ la, const double* _
   }
 }
 
-// Atom part of g: (G - <atom, G>) * atom (:1103-1108, :1125-1128), block per atom.
-__global__ void k_project_atoms(const double* __restrict__ dic, const double* __restrict__ atoms,
-                                double* __restrict__ g, size_t N) {
-  __shared__ double sh[32];
-  const size_t k = blockIdx.x;
+// Atom part of g: (G - <atom, G>) * atom (:1103-1108, :1125-1128), cluster per atom.
+__global__ void __launch_bounds__(512) k_project_atoms(const double* __restrict__ dic,
+                                                       const double* __restrict__ atoms, double* __restrict__ g,
+                                                       size_t N) {
+  __shared__ double sh[33];
+  namespace cg = cooperative_groups;
+  const cg::cluster_group c = cg::this_cluster();
+  const size_t nb = c.num_blocks(), k = blockIdx.x / nb;
+  const size_t step = nb * blockDim.x, first = c.block_rank() * (size_t)blockDim.x + threadIdx.x;
   double d = 0;
-  for (size_t j = threadIdx.x; j < N; j += blockDim.x) d += atoms[k * N + j] * dic[k * N + j];
-  d = block_sum(d, sh);
-  if (threadIdx.x == 0) sh[0] = d;
-  __syncthreads();
-  d = sh[0];
-  for (size_t j = threadIdx.x; j < N; j += blockDim.x)
-    g[k * N + j] = (dic[k * N + j] - d) * atoms[k * N + j];
+#pragma unroll 4
+  for (size_t j = first; j < N; j += step) d += atoms[k * N + j] * dic[k * N + j];
+  d = cluster_sum(d, sh);
+#pragma unroll 4
+  for (size_t j = first; j < N; j += step) g[k * N + j] = (dic[k * N + j] - d) * atoms[k * N + j];
 }
 
 __global__ void k_sum_losses(const double* __restrict__ loss, double* __restrict__ f, int P) {
@@ -645,7 +648,7 @@ template <typename T>
 struct EvalBufs {
   T *atoms, *lam, *tape_b, *tape_cb, *tape_phi, *a, *bary, *n, *gw, *buf2, *cbuf2, *v, *r, *ctmp;
   T *wa = nullptr, *wb = nullptr, *wc = nullptr, *wgrad = nullptr;
-  double *atoms64, *lam64, *gdic, *dot, *loss, *dpart;
+  double *atoms64, *lam64, *gdic, *dot, *loss, *dpart, *lossp;
   int* range;  // [P] scalings left the FP32 range (kernel domain, FP32 forms)
   uint8_t *sd = nullptr, *sw = nullptr, *stmp = nullptr;
 
@@ -673,6 +676,7 @@ struct EvalBufs {
     d(gdic, PKN);
     d(dot, P * K);
     d(dpart, P * K * n_segments(N));
+    d(lossp, P * ((N + kLossSeg - 1) / kLossSeg));
     d(loss, P);
     alloc_into(al, reinterpret_cast<void**>(&range), P * sizeof(int));
     if (wloss) {
@@ -698,6 +702,55 @@ size_t eval_bytes_t(size_t P, size_t K, size_t L, size_t N, bool log_domain, boo
 }
 
 int launch_cfg(wdl_ctx* ctx, size_t n) { return grid_for(n, 256, ctx->sm_count, 8); }
+
+// One cluster per row of `len` values (one warp for short rows).
+template <typename... Args, typename... Vals>
+int launch_rows(wdl_ctx* ctx, void (*kernel)(Args...), int rows, size_t len, cudaStream_t s, Vals... vals) {
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  const bool split = len >= kRowSplit;
+  const unsigned nb = split ? kRowBlocks : 1;
+  cfg.gridDim = dim3((unsigned)rows * nb);
+  cfg.blockDim = dim3(split ? 512 : len > 64 ? 256 : 32);
+  cfg.stream = s;
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = nb;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  WDL_CUDA_TRY(ctx, cudaLaunchKernelEx(&cfg, kernel, (Args)vals...));
+  WDL_LAUNCH_CHECK(ctx);
+  return WDL_OK;
+}
+
+// normalize_values of `rows` rows, with an optional copy in T (or of the logarithms).
+template <typename T>
+int normalise_rows(wdl_ctx* ctx, const double* in, double* out, int rows, size_t len, double exp_scale, T* cast,
+                   bool logs, cudaStream_t s) {
+  return launch_rows(ctx, k_normalise_rows<T>, rows, len, s, in, out, len, exp_scale, cast, logs ? 1 : 0);
+}
+
+// The inputs of a call: FP64 atoms and weights (normalised first when asked,
+// :562) and their copies in T (logarithms of the atoms in the log domain).
+template <typename T>
+int prepare_inputs(wdl_ctx* ctx, int P, int K, const double* atoms, const double* weights, bool normalise,
+                   bool logs, double* atoms64, double* lam64, T* atoms_t, T* lam_t, cudaStream_t s) {
+  const size_t KN = (size_t)K * ctx->N, PK = (size_t)P * K;
+  int rc;
+  if (normalise) {
+    if ((rc = normalise_rows<T>(ctx, atoms, atoms64, K, ctx->N, 0.0, atoms_t, logs, s))) return rc;
+    return normalise_rows<T>(ctx, weights, lam64, P, K, 0.0, lam_t, false, s);
+  }
+  WDL_CUDA_TRY(ctx, cudaMemcpyAsync(atoms64, atoms, KN * 8, cudaMemcpyDeviceToDevice, s));
+  WDL_CUDA_TRY(ctx, cudaMemcpyAsync(lam64, weights, PK * 8, cudaMemcpyDeviceToDevice, s));
+  if (logs) k_log_of<T><<<launch_cfg(ctx, KN), 256, 0, s>>>(atoms64, atoms_t, KN);
+  else k_cast<T><<<launch_cfg(ctx, KN), 256, 0, s>>>(atoms64, atoms_t, KN);
+  WDL_LAUNCH_CHECK(ctx);
+  k_cast<T><<<launch_cfg(ctx, PK), 256, 0, s>>>(lam64, lam_t, PK);
+  WDL_LAUNCH_CHECK(ctx);
+  return WDL_OK;
+}
 
 // Nested Sinkhorn of the Wasserstein loss (cpp/loss.h:92-154) on all P
 // barycenters at once, kernel domain, 50 inner iterations.
@@ -738,21 +791,8 @@ int gradient_both_t(wdl_ctx* ctx, int P, int K, int L, int loss_type, const doub
   const unsigned G_PKN = launch_cfg(ctx, PKN), G_PN = launch_cfg(ctx, PN),
                  G_2PKN = launch_cfg(ctx, 2 * PKN);
 
-  // Inputs: normalised FP64 copies (normalize_values, :562) and their T casts.
-  if (normalise) {
-    k_normalise_rows<<<K, 256, 0, s>>>(atoms, B.atoms64, N, 0.0);
-    WDL_LAUNCH_CHECK(ctx);
-    k_normalise_rows<<<P, 32, 0, s>>>(weights, B.lam64, K, 0.0);
-    WDL_LAUNCH_CHECK(ctx);
-  } else {
-    WDL_CUDA_TRY(ctx, cudaMemcpyAsync(B.atoms64, atoms, KN * 8, cudaMemcpyDeviceToDevice, s));
-    WDL_CUDA_TRY(ctx, cudaMemcpyAsync(B.lam64, weights, (size_t)P * K * 8, cudaMemcpyDeviceToDevice, s));
-  }
-  if (log_domain) k_log_of<T><<<launch_cfg(ctx, KN), 256, 0, s>>>(B.atoms64, B.atoms, KN);
-  else k_cast<T><<<launch_cfg(ctx, KN), 256, 0, s>>>(B.atoms64, B.atoms, KN);
-  WDL_LAUNCH_CHECK(ctx);
-  k_cast<T><<<1, 256, 0, s>>>(B.lam64, B.lam, (size_t)P * K);
-  WDL_LAUNCH_CHECK(ctx);
+  if ((rc = prepare_inputs<T>(ctx, P, K, atoms, weights, normalise, log_domain, B.atoms64, B.lam64, B.atoms, B.lam, s)))
+    return rc;
   if (b_init) {
     if (log_domain) k_log_of<T><<<G_PKN, 256, 0, s>>>(b_init, B.tape_b, PKN);
     else k_cast<T><<<G_PKN, 256, 0, s>>>(b_init, B.tape_b, PKN);
@@ -798,8 +838,11 @@ int gradient_both_t(wdl_ctx* ctx, int P, int K, int L, int loss_type, const doub
 
   // Loss and its gradient (:597).
   if (wloss && (rc = wasserstein_loss<T>(ctx, B, B.bary, observed, P, s))) return rc;
-  k_loss<T><<<P, 256, 0, s>>>(B.bary, observed, B.wgrad, B.n, B.gw, B.loss, loss_type, N);
-  WDL_LAUNCH_CHECK(ctx);
+  if ((rc = loss_segments<T>(ctx, P, B.bary, observed, B.wgrad, B.n, B.gw, B.lossp, loss_type, s))) return rc;
+  if (!wloss) {
+    k_add_segments<<<(unsigned)P, 32, 0, s>>>(B.lossp, B.loss, (int)loss_parts(ctx));
+    WDL_LAUNCH_CHECK(ctx);
+  }
 
   // Reverse pass, both recursions per round (:602-673 / :730-812).  With no
   // dictionary gradient requested, the kernel domain runs the weight
@@ -929,15 +972,7 @@ int barycenter_t(wdl_ctx* ctx, int P, int K, int L, const double* atoms, const d
   T* bary = A.take<T>(PN);
   int* range = (!log_domain && sizeof(T) == 4) ? A.take<int>((size_t)P) : nullptr;
   if (range) WDL_CUDA_TRY(ctx, cudaMemsetAsync(range, 0, (size_t)P * sizeof(int), s));
-  k_normalise_rows<<<K, 256, 0, s>>>(atoms, atoms64, N, 0.0);
-  WDL_LAUNCH_CHECK(ctx);
-  k_normalise_rows<<<P, 32, 0, s>>>(weights, lam64, K, 0.0);
-  WDL_LAUNCH_CHECK(ctx);
-  if (log_domain) k_log_of<T><<<launch_cfg(ctx, KN), 256, 0, s>>>(atoms64, at, KN);
-  else k_cast<T><<<launch_cfg(ctx, KN), 256, 0, s>>>(atoms64, at, KN);
-  WDL_LAUNCH_CHECK(ctx);
-  k_cast<T><<<1, 256, 0, s>>>(lam64, lam, (size_t)P * K);
-  WDL_LAUNCH_CHECK(ctx);
+  if ((rc = prepare_inputs<T>(ctx, P, K, atoms, weights, true, log_domain, atoms64, lam64, at, lam, s))) return rc;
   k_fill<T><<<launch_cfg(ctx, PKN), 256, 0, s>>>(b, log_domain ? T(0) : T(1), PKN);
   WDL_LAUNCH_CHECK(ctx);
   for (int it = 0; it < L; ++it) {
@@ -1002,7 +1037,7 @@ struct BandBufs {
       d(e.gdic, KN);
       d(e.dotp, P * K * band_dot_parts<T>(ctx, (int)K));
       d(e.dot, P * K);
-      d(e.lossp, P * band_loss_parts(ctx));
+      d(e.lossp, P * loss_parts(ctx));
       d(loss, P);
     }
     if (wloss) {
@@ -1029,30 +1064,21 @@ size_t band_bytes(const wdl_ctx* ctx, size_t P, size_t K, size_t L, bool b_init,
   return plan.off + 256;
 }
 
-// Kernel-domain contexts without tensor cores whose lines fit.
+// Kernel-domain contexts whose lines fit: those without tensor cores, and those
+// above the fused kernel's grids (sides over 128, volumes) whose factor is narrow
+// enough for the banded FP32 sums to beat the tensor-core axis passes.
 bool use_band(const wdl_ctx* ctx, int K) {
-  if (ctx->domain != WDL_DOMAIN_KERNEL || ctx->tc) return false;
+  if (ctx->domain != WDL_DOMAIN_KERNEL || tc_fused(ctx)) return false;
+  if (ctx->tc && !band_narrow(ctx)) return false;
   return ctx->precision == WDL_FP64 ? band_fits<double>(ctx, K) : band_fits<float>(ctx, K);
 }
 
-// Inputs: normalised FP64 copies (normalize_values, :562) and their T casts.
 template <typename T>
 int band_inputs(wdl_ctx* ctx, BandBufs<T>& B, int P, int K, const double* atoms, const double* weights,
                 bool normalise, cudaStream_t s) {
-  const size_t N = ctx->N, KN = (size_t)K * N;
-  if (normalise) {
-    k_normalise_rows<<<K, 256, 0, s>>>(atoms, B.atoms64, N, 0.0);
-    WDL_LAUNCH_CHECK(ctx);
-    k_normalise_rows<<<P, 32, 0, s>>>(weights, B.lam64, K, 0.0);
-    WDL_LAUNCH_CHECK(ctx);
-  } else {
-    WDL_CUDA_TRY(ctx, cudaMemcpyAsync(B.atoms64, atoms, KN * 8, cudaMemcpyDeviceToDevice, s));
-    WDL_CUDA_TRY(ctx, cudaMemcpyAsync(B.lam64, weights, (size_t)P * K * 8, cudaMemcpyDeviceToDevice, s));
-  }
-  k_cast<T><<<launch_cfg(ctx, KN), 256, 0, s>>>(B.atoms64, B.atoms, KN);
-  WDL_LAUNCH_CHECK(ctx);
-  k_cast<T><<<1, 256, 0, s>>>(B.lam64, B.lam, (size_t)P * K);
-  WDL_LAUNCH_CHECK(ctx);
+  int rc;
+  if ((rc = prepare_inputs<T>(ctx, P, K, atoms, weights, normalise, false, B.atoms64, B.lam64, B.atoms, B.lam, s)))
+    return rc;
   if (sizeof(T) == 4) {
     WDL_CUDA_TRY(ctx, cudaMemsetAsync(B.e.range, 0, (size_t)P * sizeof(int), s));
   } else {
@@ -1098,7 +1124,7 @@ int gradient_band_t(wdl_ctx* ctx, int P, int K, int L, int loss_type, const doub
     WDL_LAUNCH_CHECK(ctx);
   }
   if (wloss && (rc = wasserstein_loss<T>(ctx, B, bary, observed, P, s))) return rc;
-  if ((rc = band_loss<T>(ctx, e, observed, B.wgrad, loss_type, s))) return rc;
+  if ((rc = loss_segments<T>(ctx, P, bary, observed, B.wgrad, e.n, e.gw, e.lossp, loss_type, s))) return rc;
   WDL_CUDA_TRY(ctx, cudaMemsetAsync(e.dotp, 0, (size_t)P * K * band_dot_parts<T>(ctx, (int)K) * sizeof(double), s));
   if (e.dict) WDL_CUDA_TRY(ctx, cudaMemsetAsync(e.gdic, 0, KN * sizeof(double), s));
   if ((rc = band_backward<T>(ctx, e, wloss ? nullptr : B.loss, s))) return rc;
@@ -1184,20 +1210,10 @@ bool use_fused(const wdl_ctx* ctx, int loss_type) {
 
 int prepare_fused(wdl_ctx* ctx, FusedBufs& B, int P, int K, const double* atoms,
                   const double* weights, const double* b_init, bool normalise, cudaStream_t s) {
-  const size_t N = ctx->N, KN = (size_t)K * N, PKN = (size_t)P * KN;
-  if (normalise) {
-    k_normalise_rows<<<K, 256, 0, s>>>(atoms, B.atoms64, N, 0.0);
-    WDL_LAUNCH_CHECK(ctx);
-    k_normalise_rows<<<P, 32, 0, s>>>(weights, B.lam64, K, 0.0);
-    WDL_LAUNCH_CHECK(ctx);
-  } else {
-    WDL_CUDA_TRY(ctx, cudaMemcpyAsync(B.atoms64, atoms, KN * 8, cudaMemcpyDeviceToDevice, s));
-    WDL_CUDA_TRY(ctx, cudaMemcpyAsync(B.lam64, weights, (size_t)P * K * 8, cudaMemcpyDeviceToDevice, s));
-  }
-  k_cast<float><<<launch_cfg(ctx, KN), 256, 0, s>>>(B.atoms64, B.atoms, KN);
-  WDL_LAUNCH_CHECK(ctx);
-  k_cast<float><<<1, 256, 0, s>>>(B.lam64, B.lam, (size_t)P * K);
-  WDL_LAUNCH_CHECK(ctx);
+  const size_t PKN = (size_t)P * K * ctx->N;
+  int rc;
+  if ((rc = prepare_inputs<float>(ctx, P, K, atoms, weights, normalise, false, B.atoms64, B.lam64, B.atoms, B.lam, s)))
+    return rc;
   if (b_init) {
     k_cast<float><<<launch_cfg(ctx, PKN), 256, 0, s>>>(b_init, B.b0, PKN);
     WDL_LAUNCH_CHECK(ctx);
@@ -1475,17 +1491,14 @@ int evaluate_both_dev(wdl_ctx* ctx, int P, int K, int L, int loss_type, double s
   double* dic = carve(KN);
   double* loss = carve(P);
   // Back to the original domain and normalise (:997-1031).
-  k_normalise_rows<<<P, 32, 0, s>>>(x, w2, K, scale_dic);
-  WDL_LAUNCH_CHECK(ctx);
-  k_normalise_rows<<<K, 256, 0, s>>>(x + PK, a2, N, 1.0);
-  WDL_LAUNCH_CHECK(ctx);
+  if ((rc = normalise_rows<double>(ctx, x, w2, P, K, scale_dic, nullptr, false, s))) return rc;
+  if ((rc = normalise_rows<double>(ctx, x + PK, a2, K, N, 1.0, nullptr, false, s))) return rc;
   if ((rc = gradient_both_dev(ctx, P, K, L, loss_type, a2, w2, observed, b_storage, la, dic, bary,
                               loss, b_last, s, true)))
     return rc;
   k_project_weights<<<grid_for(P, 128, ctx->sm_count), 128, 0, s>>>(la, w2, g, P, K, scale_dic);
   WDL_LAUNCH_CHECK(ctx);
-  k_project_atoms<<<K, 256, 0, s>>>(dic, a2, g + PK, N);
-  WDL_LAUNCH_CHECK(ctx);
+  if ((rc = launch_rows(ctx, k_project_atoms, K, N, s, dic, a2, g + PK, N))) return rc;
   k_sum_losses<<<1, 32, 0, s>>>(loss, f, P);
   WDL_LAUNCH_CHECK(ctx);
   return WDL_OK;

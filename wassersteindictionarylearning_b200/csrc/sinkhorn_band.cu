@@ -20,16 +20,20 @@
 //
 // Against dense axis passes (64 x 64 tiles, all C taps) with separate
 // elementwise kernels, one B200: 64 histograms of 128 x 128, K = 5, L = 100,
-// gamma 1, FP32 69.3 -> 24.5 ms an evaluation; 16 of 64 x 64, K = 4, L = 25, FP32
-// 2.38 -> 0.96 ms (350 -> 100 launches); one of 161 x 161, K = 5, L = 50, FP64,
-// weights only 10.9 -> 2.3 ms.  The dense passes spent 128 taps where 13 reach
-// the FP32 rounding; here the kernels are bound by issue (55-60 % of the slots
-// at 128 x 128) and, for few histograms, by each launch's latency.
+// gamma 1, FP32 69.4 -> 20.3 ms an evaluation; 16 of 64 x 64, K = 4, L = 25, FP32
+// 2.38 -> 0.84 ms (350 -> 100 launches); one of 161 x 161, K = 5, L = 50, FP64,
+// weights only 10.9 -> 2.2 ms.  The dense passes spent 128 taps where 13 reach
+// the FP32 rounding; here the kernels are bound by issue (a quarter of the
+// instructions at 128 x 128 are the sums' packed multiply-adds, the rest the
+// logarithms, divisions, staging and addresses) and, for few histograms, by each
+// launch's latency.  Tiles that lie inside the image and are whole groups of eight
+// take a form without edge tests (24.4 -> 21.4 ms at 128 x 128).
 //
 // The blocks' shapes depend on the grid, K and the type only, so a
 // histogram's results are the same bits in any batch.
 #include <algorithm>
 #include <cmath>
+#include <type_traits>
 
 #include "band.cuh"
 #include "wdl_internal.cuh"
@@ -42,6 +46,7 @@ using namespace band;
 
 constexpr int kMaxThreads = 256, kMaxWarps = kMaxThreads / 32;
 constexpr size_t kSmemMost = 200 * 1024;
+constexpr int kMaxK = 64;  // atoms of one rows block
 
 template <typename T>
 const T* factor_row(const wdl_ctx* ctx, int axis);
@@ -92,6 +97,15 @@ size_t band_smem(const Axis<T>& ax, int blocks, int lines) {
 }
 
 // ---- shared pieces ------------------------------------------------------------------
+// The kernels of an evaluation depend on one another in a chain.  Each lets the
+// next one start once all its own blocks run, so that the next one's first
+// blocks fill the SMs that the last blocks leave idle and have their tables
+// ready; wait_previous then holds them until everything the chain wrote before
+// is visible.  No global memory that another kernel of the chain touches is
+// read or written before it.
+__device__ __forceinline__ void start_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void wait_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // W global rows (contiguous, src0 and src1) into one zero-padded SMEM line, by one
 // warp; m takes their magnitudes.  No input: ones.  Rows of whole 16-byte units
 // are read four values at a time.
@@ -138,8 +152,8 @@ __device__ __forceinline__ void fill_row(typename Vec<T>::V* dst, const TI* __re
   }
 }
 
-// Eight consecutive values of one of the interleaved rows to global memory
-// (C % 4 == 0: 16-byte stores).
+// Eight consecutive values of one of the interleaved rows to global memory; FULL:
+// whole 16-byte units, all eight inside the row.
 __device__ __forceinline__ void put4(float* p, const float* v) {
   *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
 }
@@ -147,37 +161,33 @@ __device__ __forceinline__ void put4(double* p, const double* v) {
   *reinterpret_cast<double2*>(p) = make_double2(v[0], v[1]);
   *reinterpret_cast<double2*>(p + 2) = make_double2(v[2], v[3]);
 }
-template <typename T>
+template <bool FULL, typename T>
 __device__ __forceinline__ void store_row8(T* __restrict__ dst, int c0, int C, const T (&v)[8]) {
-  if ((C & 3) == 0) {
+  if (FULL) {
     put4(dst, v);
-    if (c0 + 4 < C) put4(dst + 4, v + 4);
+    put4(dst + 4, v + 4);
   } else {
 #pragma unroll
     for (int j = 0; j < 8; ++j)
       if (c0 + j < C) dst[j] = v[j];
   }
 }
-template <typename T>
-__device__ __forceinline__ void component(const typename Vec<T>::V (&acc)[8], int c, T (&v)[8]) {
+// Outputs of a row item to rows r, r + 1 (those below `rows`) of an image.
+template <bool FULL, typename T>
+__device__ __forceinline__ void store_rows(T* __restrict__ img, int r, int rows, int c0, int C,
+                                           const typename Vec<T>::V (&acc)[8]) {
+  T v[Vec<T>::W][8];
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
     T t[Vec<T>::W];
     Vec<T>::split(acc[j], t);
-    v[j] = t[c];
-  }
-}
-// Outputs of a row item to rows r, r + 1 (those below `rows`) of an image.
-template <typename T>
-__device__ __forceinline__ void store_rows(T* __restrict__ img, int r, int rows, int c0, int C,
-                                           const typename Vec<T>::V (&acc)[8]) {
 #pragma unroll
-  for (int c = 0; c < Vec<T>::W; ++c) {
-    if (r + c >= rows) continue;
-    T v[8];
-    component<T>(acc, c, v);
-    store_row8(img + (size_t)(r + c) * C + c0, c0, C, v);
+    for (int c = 0; c < Vec<T>::W; ++c) v[c][j] = t[c];
   }
+  T* d = img + (uint32_t)(r * C + c0);
+#pragma unroll
+  for (int c = 0; c < Vec<T>::W; ++c)
+    if (FULL || r + c < rows) store_row8<FULL>(d + c * C, c0, C, v[c]);
 }
 
 template <typename T>
@@ -185,10 +195,17 @@ struct NoExt {
   __device__ void operator()(int, int, T (&)[1][8][Vec<T>::W]) const {}
 };
 
+// Lines past the last row repeat it (their results are dropped): every block
+// has the same number of lines, and a repeated line changes no other's radius.
+template <typename T>
+__device__ __forceinline__ const T* row_at(const T* img, int r, int rows, int C) {
+  return img + (uint32_t)(min(r, rows - 1) * C);
+}
+
 // ---- the operator alone: x pass over rows ---------------------------------------------
 template <typename TI, typename T>
-__global__ void __launch_bounds__(kMaxThreads) k_rows_op(Axis<T> ax, const TI* __restrict__ in,
-                                                         T* __restrict__ out, int rows, int n) {
+__global__ void __launch_bounds__(kMaxThreads, 3) k_rows_op(Axis<T> ax, const TI* __restrict__ in,
+                                                         T* __restrict__ out, int rows, Div n) {
   using V = typename Vec<T>::V;
   constexpr int W = Vec<T>::W;
   extern __shared__ __align__(16) unsigned char smem[];
@@ -196,76 +213,92 @@ __global__ void __launch_bounds__(kMaxThreads) k_rows_op(Axis<T> ax, const TI* _
   V* S = tab + table_elems(ax) + kPad;
   __shared__ int mag[kMaxWarps];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nt = blockDim.x, nw = nt >> 5;
-  const int r0 = blockIdx.x * n * W, nl = min(n, (rows - r0 + W - 1) / W), C = ax.C;
+  const int r0 = blockIdx.x * n.n * W, C = ax.C;
   const size_t base = (size_t)blockIdx.y * rows * C;
+  start_next();
   const V* g = load_table(ax, tab, tid, nt);
-  zero_pads(ax, S, nl, tid, nt);
+  zero_pads(ax, S, n.n, tid, nt);
+  wait_previous();
   typename Vec<T>::M m = 0;
-  for (int l = warp; l < nl; l += nw) {
+  for (int l = warp; l < n.n; l += nw) {
     const int r = r0 + l * W;
-    const TI* s = in ? in + base + (size_t)r * C : nullptr;
-    fill_row<T>(S + l * ax.pitch, s, in && r + 1 < rows ? s + C : s, ax, lane, m);
+    const TI* s0 = in ? row_at(in + base, r, rows, C) : nullptr;
+    fill_row<T>(S + l * ax.pitch, s0, in ? row_at(in + base, r + 1, rows, C) : nullptr, ax, lane, m);
   }
   put_mag<T>(mag, m, warp, lane);
   __syncthreads();
-  fir_lines<T, 0>(S, g, ax, nl, div_magic(nl), get_mag(mag, nw, lane), warp, nw, lane, NoExt<T>(),
-                  [&](int l, int c0, const V(&acc)[8], const T(&)[1][8][W]) {
-                    store_rows<T>(out + base, r0 + l * W, rows, c0, C, acc);
-                  });
+  const bool full = (C & 7) == 0 && r0 + n.n * W <= rows;
+  const auto run = [&](auto f) {
+    fir_lines<T, 0>(S, g, ax, n, get_mag(mag, nw, lane), warp, nw, lane, NoExt<T>(),
+                    [&](int l, int c0, const V(&acc)[8], const T(&)[1][8][W]) {
+                      store_rows<decltype(f)::value>(out + base, r0 + l * W, rows, c0, C, acc);
+                    });
+  };
+  if (full) run(std::true_type());
+  else run(std::false_type());
 }
 
 // ---- forward rows ---------------------------------------------------------------------
 // x pass of t2 -> phi (stored); bary = exp(sum_k lambda_k log phi_k) (stored);
 // b = bary / phi -> x pass -> t1 (cpp/inverseWasserstein.h:575-593).  t1 null:
 // the last iteration.  Lines: atom by atom, the block's row groups of each.
-template <typename T, int KT>
-__global__ void __launch_bounds__(kMaxThreads) k_rows_fwd(Axis<T> ax, const T* __restrict__ t2,
-                                                          const double* __restrict__ lam, T* __restrict__ phi,
-                                                          T* __restrict__ bary, T* __restrict__ t1,
-                                                          int* __restrict__ range, int K_, int rows, int n,
-                                                          int nchunk) {
+template <typename T>
+struct FwdRows {
+  const T* t2;
+  const double* lam;
+  T *phi, *bary, *t1;
+  int* range;
+  int K, rows, nchunk;
+  Div nv, nl, C;  // row groups of an atom, lines of the block, row length
+};
+
+template <typename T, int KT, bool FULL>
+__device__ __forceinline__ void rows_fwd(const Axis<T>& ax, const FwdRows<T>& a, int p, int r0,
+                                         typename Vec<T>::V* tab, int (*mag)[kMaxWarps], double* slam) {
   using V = typename Vec<T>::V;
   constexpr int W = Vec<T>::W;
-  const int K = KT > 0 ? KT : K_;
-  extern __shared__ __align__(16) unsigned char smem[];
-  V* tab = reinterpret_cast<V*>(smem);
-  V* S1 = tab + table_elems(ax) + kPad;
-  V* S2 = S1 + lines_elems(ax, K * n);
-  __shared__ int mag[2][kMaxWarps];
+  const int K = KT > 0 ? KT : a.K;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nt = blockDim.x, nw = nt >> 5;
-  const int p = blockIdx.x / nchunk, r0 = (blockIdx.x - p * nchunk) * n * W;
-  const int C = ax.C, nv = min(n, (rows - r0 + W - 1) / W), nl = K * nv;
-  const uint32_t inv_nv = div_magic(nv), inv_nl = div_magic(nl), inv_C = div_magic(C);
-  const size_t N = (size_t)rows * C, pN = (size_t)p * N;
+  const int C = ax.C, rows = a.rows, nv = a.nv.n, nl = a.nl.n;
+  const uint32_t N = (uint32_t)rows * C;
+  const size_t pN = (size_t)p * N;
+  V* S1 = tab + table_elems(ax) + kPad;
+  V* S2 = S1 + lines_elems(ax, nl);
   const V* g = load_table(ax, tab, tid, nt);
   zero_pads(ax, S1, nl, tid, nt);
+  wait_previous();
+  for (int k = tid; k < K; k += nt) slam[k] = a.lam[(size_t)p * K + k];
   typename Vec<T>::M m = 0;
+  const T* t2 = a.t2 + pN * K;
   for (int l = warp; l < nl; l += nw) {
-    const int k = fast_div(l, nv, inv_nv), r = r0 + (l - k * nv) * W;
-    const T* s = t2 + (pN * K + k * N) + (size_t)r * C;
-    fill_row<T>(S1 + l * ax.pitch, s, r + 1 < rows ? s + C : s, ax, lane, m);
+    const int k = a.nv(l), r = r0 + (l - k * nv) * W;
+    fill_row<T>(S1 + l * ax.pitch, row_at(t2 + k * N, r, rows, C), row_at(t2 + k * N, r + 1, rows, C), ax, lane, m);
   }
   put_mag<T>(mag[0], m, warp, lane);
   __syncthreads();
-  fir_lines<T, 0>(S1, g, ax, nl, inv_nl, get_mag(mag[0], nw, lane), warp, nw, lane, NoExt<T>(),
+  fir_lines<T, 0>(S1, g, ax, a.nl, get_mag(mag[0], nw, lane), warp, nw, lane, NoExt<T>(),
                   [&](int l, int c0, const V(&acc)[8], const T(&)[1][8][W]) { st8(S2 + l * ax.pitch + c0, acc); });
   __syncthreads();
   m = 0;
+  const int kstep = nv * ax.pitch;
   for (int e = tid; e < nv * C; e += nt) {
-    const int v = fast_div(e, C, inv_C), x = e - v * C, r = r0 + v * W;
-    const size_t j = pN + (size_t)r * C + x;
+    const int v = a.C(e), x = e - v * C, r = r0 + v * W;
+    const uint32_t j = (uint32_t)(min(r, rows - 1) * C + x);
+    const bool ok0 = FULL || r < rows, ok1 = FULL || r + 1 < rows;
+    V* s2 = S2 + v * ax.pitch + x;
+    V* s1 = S1 + v * ax.pitch + x;
+    T* pp = a.phi ? a.phi + pN * K + j : nullptr;
     double s[W];
 #pragma unroll
     for (int c = 0; c < W; ++c) s[c] = 0;
 #pragma unroll
     for (int k = 0; k < K; ++k) {
       T ph[W];
-      Vec<T>::split(S2[(k * nv + v) * ax.pitch + x], ph);
-      const double l = lam[(size_t)p * K + k];
-      T* pp = phi ? phi + (j + pN * (K - 1) + k * N) : nullptr;
+      Vec<T>::split(s2[k * kstep], ph);
+      const double l = slam[k];
 #pragma unroll
       for (int c = 0; c < W; ++c) {
-        if (pp && r + c < rows) pp[c * C] = ph[c];
+        if (pp && (c ? ok1 : ok0)) pp[k * N + c * C] = ph[c];
         s[c] += acc_safe_log<T>(ph[c]) * l;
       }
     }
@@ -273,30 +306,40 @@ __global__ void __launch_bounds__(kMaxThreads) k_rows_fwd(Axis<T> ax, const T* _
 #pragma unroll
     for (int c = 0; c < W; ++c) {
       by[c] = exp_from<T>(s[c]);
-      if (bary && r + c < rows) bary[j + c * C] = by[c];
+      if (a.bary && (c ? ok1 : ok0)) (a.bary + pN)[j + c * C] = by[c];
     }
 #pragma unroll
     for (int k = 0; k < K; ++k) {
-      const int o = (k * nv + v) * ax.pitch + x;
       T b[W];
-      Vec<T>::split(S2[o], b);
+      Vec<T>::split(s2[k * kstep], b);
 #pragma unroll
-      for (int c = 0; c < W; ++c) {
-        b[c] = by[c] / b[c];
-      }
+      for (int c = 0; c < W; ++c) b[c] = by[c] / b[c];
       m = Vec<T>::up(m, b);
-      S1[o] = Vec<T>::make(b);
+      s1[k * kstep] = Vec<T>::make(b);
     }
   }
-  if (range && !Vec<T>::finite(m)) range[p] = 1;
-  if (!t1) return;
+  if (a.range && !Vec<T>::finite(m)) a.range[p] = 1;
+  if (!a.t1) return;
   put_mag<T>(mag[1], m, warp, lane);
   __syncthreads();
-  fir_lines<T, 0>(S1, g, ax, nl, inv_nl, get_mag(mag[1], nw, lane), warp, nw, lane, NoExt<T>(),
+  T* t1 = a.t1 + pN * K;
+  fir_lines<T, 0>(S1, g, ax, a.nl, get_mag(mag[1], nw, lane), warp, nw, lane, NoExt<T>(),
                   [&](int l, int c0, const V(&acc)[8], const T(&)[1][8][W]) {
-                    const int k = fast_div(l, nv, inv_nv), r = r0 + (l - k * nv) * W;
-                    store_rows<T>(t1 + (pN * K + k * N), r, rows, c0, C, acc);
+                    const int k = a.nv(l), r = r0 + (l - k * nv) * W;
+                    store_rows<FULL>(t1 + k * N, r, rows, c0, C, acc);
                   });
+}
+
+template <typename T, int KT>
+__global__ void __launch_bounds__(kMaxThreads, 3) k_rows_fwd(Axis<T> ax, FwdRows<T> a) {
+  start_next();
+  extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ int mag[2][kMaxWarps];
+  __shared__ double slam[kMaxK];
+  const int p = blockIdx.x / a.nchunk, r0 = (blockIdx.x - p * a.nchunk) * a.nv.n * Vec<T>::W;
+  auto* tab = reinterpret_cast<typename Vec<T>::V*>(smem);
+  if ((ax.C & 7) == 0 && r0 + a.nv.n * Vec<T>::W <= a.rows) rows_fwd<T, KT, true>(ax, a, p, r0, tab, mag, slam);
+  else rows_fwd<T, KT, false>(ax, a, p, r0, tab, mag, slam);
 }
 
 // ---- reverse rows -----------------------------------------------------------------------
@@ -313,69 +356,55 @@ struct BwdRows {
   const T *t2, *n, *gw, *phi, *bary, *lam;
   T* t1;
   double* dotp;
-  int K, P, rows, nv, nchunk, nblocks, dict, want_u;
+  int K, P, rows, nchunk, nblocks, dict, want_u;
+  Div nv, nl, C;
   size_t PKN;
   const T* q;
   double* gdic;
 };
 
-template <typename T, int KT, bool FIRST>
-__global__ void __launch_bounds__(kMaxThreads) k_rows_bwd(Axis<T> ax, BwdRows<T> a) {
+template <typename T, int KT, bool FIRST, bool FULL>
+__device__ __forceinline__ void rows_bwd(const Axis<T>& ax, const BwdRows<T>& a, int p, int r0,
+                                         typename Vec<T>::V* tab, int (*mag)[kMaxWarps], T* slam) {
   using V = typename Vec<T>::V;
   constexpr int W = Vec<T>::W, KR = KT > 0 ? KT : 1;
   const int K = KT > 0 ? KT : a.K;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nt = blockDim.x, nw = nt >> 5;
-  const int rows = a.rows, C = ax.C;
-  const size_t N = (size_t)rows * C, KN = (size_t)K * N;
-  if ((int)blockIdx.x >= a.nblocks) {
-    const size_t step = (size_t)(gridDim.x - a.nblocks) * nt;
-    for (size_t i = (size_t)(blockIdx.x - a.nblocks) * nt + tid; i < KN; i += step) {
-      double s = 0;
-#pragma unroll 8
-      for (int p = 0; p < a.P; ++p) s += (double)a.q[(size_t)p * KN + i];
-      a.gdic[i] += s;
-    }
-    return;
-  }
-  extern __shared__ __align__(16) unsigned char smem[];
-  V* tab = reinterpret_cast<V*>(smem);
-  V* S1 = tab + table_elems(ax) + kPad;                // [dictionary, weights][K * n] lines
-  const int half = K * a.nv * ax.pitch;                // from the dictionary's lines to the weights'
-  V* S2 = S1 + lines_elems(ax, 2 * K * a.nv);          // the same
-  double* sdot = reinterpret_cast<double*>(S2 + 2 * half);  // [warp][K]
-  __shared__ int mag[4][kMaxWarps];
-  const int p = blockIdx.x / a.nchunk, chunk = blockIdx.x - p * a.nchunk, r0 = chunk * a.nv * W;
-  const int nv = min(a.nv, (rows - r0 + W - 1) / W), nl = K * nv;
-  const uint32_t inv_nv = div_magic(nv), inv_nl = div_magic(nl), inv_C = div_magic(C);
+  const int rows = a.rows, C = ax.C, nv = a.nv.n, nl = a.nl.n;
+  const uint32_t N = (uint32_t)rows * C;
   const size_t pN = (size_t)p * N;
+  V* S1 = tab + table_elems(ax) + kPad;                // [dictionary, weights][K * n] lines
+  const int half = nl * ax.pitch;                      // from the dictionary's lines to the weights'
+  V* S2 = S1 + lines_elems(ax, 2 * nl);                // the same
+  double* sdot = reinterpret_cast<double*>(S2 + 2 * half);  // [warp][K]
   const int q0 = a.dict ? 0 : 1;
   // the weights' items start on the warp after the dictionary's last
   const int warp_w = a.dict ? (warp + nw - ((nl * ax.G + 31) >> 5) % nw) % nw : warp;
   const V* g = load_table(ax, tab, tid, nt);
   for (int q = q0; q < 2; ++q) zero_pads(ax, S1 + q * half, nl, tid, nt);
+  wait_previous();
+  for (int k = tid; k < K; k += nt) slam[k] = a.lam[(size_t)p * K + k];
+  if (KT == 0)
+    for (int i = tid; i < nw * K; i += nt) sdot[i] = 0;
   if (!FIRST) {
-    for (int q = q0; q < 2; ++q) {
-      typename Vec<T>::M m = 0;
-      for (int l = warp; l < nl; l += nw) {
-        const int k = fast_div(l, nv, inv_nv), r = r0 + (l - k * nv) * W;
-        const T* s = a.t2 + (q * a.PKN + pN * K + k * N) + (size_t)r * C;
-        fill_row<T>(S1 + q * half + l * ax.pitch, s, r + 1 < rows ? s + C : s, ax, lane, m);
-      }
-      put_mag<T>(mag[q], m, warp, lane);
+    typename Vec<T>::M m[2] = {0, 0};
+    for (int l2 = (q0 ? nl : 0) + warp; l2 < 2 * nl; l2 += nw) {
+      const int q = l2 >= nl ? 1 : 0, l = l2 - q * nl;
+      const int k = a.nv(l), r = r0 + (l - k * nv) * W;
+      const T* t2 = a.t2 + (q * a.PKN + pN * K) + k * N;
+      fill_row<T>(S1 + q * half + l * ax.pitch, row_at(t2, r, rows, C), row_at(t2, r + 1, rows, C), ax, lane, m[q]);
     }
-    if (KT == 0)
-      for (int i = tid; i < nw * K; i += nt) sdot[i] = 0;
+    put_mag<T>(mag[0], m[0], warp, lane);
+    put_mag<T>(mag[1], m[1], warp, lane);
     __syncthreads();
     for (int q = q0; q < 2; ++q)
-      fir_lines<T, 0>(S1 + q * half, g, ax, nl, inv_nl, get_mag(mag[q], nw, lane), q ? warp_w : warp, nw, lane,
-                      NoExt<T>(), [&](int l, int c0, const V(&acc)[8], const T(&)[1][8][W]) {
+      fir_lines<T, 0>(S1 + q * half, g, ax, a.nl, get_mag(mag[q], nw, lane), q ? warp_w : warp, nw, lane, NoExt<T>(),
+                      [&](int l, int c0, const V(&acc)[8], const T(&)[1][8][W]) {
                         st8(S2 + q * half + l * ax.pitch + c0, acc);
                       });
     __syncthreads();
   } else {
-    if (KT == 0)
-      for (int i = tid; i < nw * K; i += nt) sdot[i] = 0;
-    if (C < ax.C8)  // the lines' ends
+    if (!FULL)  // the lines' ends
       for (int i = tid; i < 2 * nl * 8; i += nt) {
         const int l = i >> 3, x = ax.C8 - 8 + (i & 7);
         if (x >= C) S1[l < nl ? l * ax.pitch + x : half + (l - nl) * ax.pitch + x] = 0;
@@ -386,78 +415,76 @@ __global__ void __launch_bounds__(kMaxThreads) k_rows_bwd(Axis<T> ax, BwdRows<T>
   double dot[KR];
 #pragma unroll
   for (int k = 0; k < KR; ++k) dot[k] = 0;
+  const int kstep = nv * ax.pitch;
+  const T* phi = a.phi + pN * K;
+  const T* bary = a.bary + pN;
   for (int e0 = warp * 32; e0 < nv * C; e0 += nt) {
-    const bool ok = e0 + lane < nv * C;
-    const int e = ok ? e0 + lane : 0;
-    const int v = fast_div(e, C, inv_C), x = e - v * C, r = r0 + v * W;
-    const int up = W > 1 && r + 1 < rows ? C : 0;  // from the first row to the second
-    const size_t j = (size_t)r * C + x;
+    const bool in = e0 + lane < nv * C;
+    const int e = in ? e0 + lane : 0;
+    const int v = a.C(e), x = e - v * C, r = r0 + v * W;
+    const bool ok0 = in && (FULL || r < rows), ok1 = in && (FULL || r + 1 < rows);
+    const uint32_t up = FULL || r + 1 < rows ? C : 0;  // from the first row to the second
+    const uint32_t j = (uint32_t)((FULL ? r : min(r, rows - 1)) * C + x);
+    V* s1 = S1 + v * ax.pitch + x;
+    V* s2 = S2 + v * ax.pitch + x;
     T ph[KR][W], bk[KR][W], by[W], sn[W], sg[W];
-    const T* php = a.phi + (pN * K + j);
 #pragma unroll
     for (int c = 0; c < W; ++c) {
-      by[c] = a.bary[pN + j + c * up];
+      by[c] = bary[j + c * up];
       if (KT > 0) {
 #pragma unroll
-        for (int k = 0; k < KR; ++k) ph[k][c] = php[k * N + c * up];
+        for (int k = 0; k < KR; ++k) ph[k][c] = phi[k * N + j + c * up];
       }
-      sn[c] = FIRST && a.dict ? a.n[pN + j + c * up] : T(0);
-      sg[c] = FIRST ? a.gw[pN + j + c * up] : T(0);
+      sn[c] = FIRST && a.dict ? (a.n + pN)[j + c * up] : T(0);
+      sg[c] = FIRST ? (a.gw + pN)[j + c * up] : T(0);
     }
 #pragma unroll
     for (int k = 0; k < K; ++k) {
-      const int o = (k * nv + v) * ax.pitch + x;
       T h[W], b[W], vv[W], rv[W];
 #pragma unroll
       for (int c = 0; c < W; ++c) {
-        h[c] = KT > 0 ? ph[KT > 0 ? k : 0][c] : php[k * N + c * up];
+        h[c] = KT > 0 ? ph[KT > 0 ? k : 0][c] : phi[k * N + j + c * up];
         b[c] = by[c] / h[c];
         if (KT > 0) bk[KT > 0 ? k : 0][c] = b[c];
       }
-      if (!FIRST && ok) {
+      if (!FIRST && in) {
         if (a.dict) {
-          Vec<T>::split(S2[o], vv);
+          Vec<T>::split(s2[k * kstep], vv);
 #pragma unroll
           for (int c = 0; c < W; ++c) sn[c] += vv[c] /= h[c];
-          S2[o] = Vec<T>::make(vv);
+          s2[k * kstep] = Vec<T>::make(vv);
         }
-        Vec<T>::split(S2[half + o], rv);
+        Vec<T>::split(s2[half + k * kstep], rv);
 #pragma unroll
         for (int c = 0; c < W; ++c) sg[c] += rv[c] *= b[c];
-        S2[half + o] = Vec<T>::make(rv);
+        s2[half + k * kstep] = Vec<T>::make(rv);
       }
     }
 #pragma unroll
     for (int k = 0; k < K; ++k) {
-      const int o = (k * nv + v) * ax.pitch + x;
-      const T l = a.lam[(size_t)p * K + k];
+      const T l = slam[k];
       T h[W], b[W], t[W], u[W];
       double acc = 0;
 #pragma unroll
       for (int c = 0; c < W; ++c) {
-        h[c] = KT > 0 ? ph[KT > 0 ? k : 0][c] : php[k * N + c * up];
+        h[c] = KT > 0 ? ph[KT > 0 ? k : 0][c] : phi[k * N + j + c * up];
         b[c] = KT > 0 ? bk[KT > 0 ? k : 0][c] : by[c] / h[c];
         t[c] = u[c] = T(0);
-        if (c == 0 || up) acc += acc_log<T>(h[c]) * (double)sg[c];
+        if (c ? ok1 : ok0) acc += acc_log<T>(h[c]) * (double)sg[c];
       }
-      if (!ok) acc = 0;
-      if (ok && a.dict) {
-        if (!FIRST) Vec<T>::split(S2[o], t);
+      if (in && a.dict) {
+        if (!FIRST) Vec<T>::split(s2[k * kstep], t);
 #pragma unroll
-        for (int c = 0; c < W; ++c) {
-          t[c] = (l * sn[c] - t[c]) * b[c];
-        }
+        for (int c = 0; c < W; ++c) t[c] = (l * sn[c] - t[c]) * b[c];
         md = Vec<T>::up(md, t);
-        S1[o] = Vec<T>::make(t);
+        s1[k * kstep] = Vec<T>::make(t);
       }
-      if (ok && a.want_u) {
-        if (!FIRST) Vec<T>::split(S2[half + o], u);
+      if (in && a.want_u) {
+        if (!FIRST) Vec<T>::split(s2[half + k * kstep], u);
 #pragma unroll
-        for (int c = 0; c < W; ++c) {
-          u[c] = (l * sg[c] - u[c]) / h[c];
-        }
+        for (int c = 0; c < W; ++c) u[c] = (l * sg[c] - u[c]) / h[c];
         mw = Vec<T>::up(mw, u);
-        S1[half + o] = Vec<T>::make(u);
+        s1[half + k * kstep] = Vec<T>::make(u);
       }
       if (KT > 0) {
         dot[KT > 0 ? k : 0] += acc;
@@ -480,17 +507,44 @@ __global__ void __launch_bounds__(kMaxThreads) k_rows_bwd(Axis<T> ax, BwdRows<T>
   put_mag<T>(mag[2], md, warp, lane);
   put_mag<T>(mag[3], mw, warp, lane);
   __syncthreads();
+  const int chunk = r0 / (nv * W);
   for (int k = tid; k < K; k += nt) {
     double s = 0;
     for (int w = 0; w < nw; ++w) s += sdot[w * K + k];
     a.dotp[((size_t)p * K + k) * a.nchunk + chunk] += s;
   }
-  for (int q = q0; q < (a.want_u ? 2 : 1); ++q)
-    fir_lines<T, 0>(S1 + q * half, g, ax, nl, inv_nl, get_mag(mag[2 + q], nw, lane), q ? warp_w : warp, nw, lane,
-                    NoExt<T>(), [&](int l, int c0, const V(&acc)[8], const T(&)[1][8][W]) {
-                      const int k = fast_div(l, nv, inv_nv), r = r0 + (l - k * nv) * W;
-                      store_rows<T>(a.t1 + (q * a.PKN + pN * K + k * N), r, rows, c0, C, acc);
+  for (int q = q0; q < (a.want_u ? 2 : 1); ++q) {
+    T* t1 = a.t1 + (q * a.PKN + pN * K);
+    fir_lines<T, 0>(S1 + q * half, g, ax, a.nl, get_mag(mag[2 + q], nw, lane), q ? warp_w : warp, nw, lane, NoExt<T>(),
+                    [&](int l, int c0, const V(&acc)[8], const T(&)[1][8][W]) {
+                      const int k = a.nv(l), r = r0 + (l - k * nv) * W;
+                      store_rows<FULL>(t1 + k * N, r, rows, c0, C, acc);
                     });
+  }
+}
+
+template <typename T, int KT, bool FIRST>
+__global__ void __launch_bounds__(kMaxThreads, 3) k_rows_bwd(Axis<T> ax, BwdRows<T> a) {
+  const int nt = blockDim.x;
+  start_next();
+  if ((int)blockIdx.x >= a.nblocks) {
+    wait_previous();
+    const size_t KN = (size_t)(KT > 0 ? KT : a.K) * a.rows * ax.C, step = (size_t)(gridDim.x - a.nblocks) * nt;
+    for (size_t i = (size_t)(blockIdx.x - a.nblocks) * nt + threadIdx.x; i < KN; i += step) {
+      double s = 0;
+#pragma unroll 8
+      for (int p = 0; p < a.P; ++p) s += (double)a.q[(size_t)p * KN + i];
+      a.gdic[i] += s;
+    }
+    return;
+  }
+  extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ int mag[4][kMaxWarps];
+  __shared__ T slam[kMaxK];
+  const int p = blockIdx.x / a.nchunk, r0 = (blockIdx.x - p * a.nchunk) * a.nv.n * Vec<T>::W;
+  auto* tab = reinterpret_cast<typename Vec<T>::V*>(smem);
+  if ((ax.C & 7) == 0 && r0 + a.nv.n * Vec<T>::W <= a.rows) rows_bwd<T, KT, FIRST, true>(ax, a, p, r0, tab, mag, slam);
+  else rows_bwd<T, KT, FIRST, false>(ax, a, p, r0, tab, mag, slam);
 }
 
 // ---- columns -----------------------------------------------------------------------------
@@ -509,15 +563,16 @@ struct Cols {
   const T *atoms, *cbr;  // [K][N]; conv_b read by kMid
   T *cb, *q;             // conv_b written by kDiv (or null); c / conv_b
   int* range;
-  int inner, chunks, n, K, PK, im0;  // images im0, im0 + 1, ...
+  int inner, chunks, K, PK, im0;  // images im0, im0 + 1, ...
+  Div n;
   size_t N;
 };
 
-// W neighbouring values of a row of the tile; pair: 8-byte accesses (an even row
-// length), up: distance to the second one (0 where there is none).
-template <typename T>
-__device__ __forceinline__ void get_cols(const T* __restrict__ p, bool pair, int up, T (&v)[Vec<T>::W]) {
-  if (Vec<T>::W == 2 && pair) {
+// W neighbouring values of a row of the tile.  FULL: both inside, 8-byte
+// accesses; else up is the distance to the second one (0 where there is none).
+template <bool FULL, typename T>
+__device__ __forceinline__ void get_cols(const T* __restrict__ p, int up, T (&v)[Vec<T>::W]) {
+  if (Vec<T>::W == 2 && FULL) {
     const float2 f = *reinterpret_cast<const float2*>(p);
     v[0] = (T)f.x;
     v[Vec<T>::W - 1] = (T)f.y;
@@ -526,48 +581,48 @@ __device__ __forceinline__ void get_cols(const T* __restrict__ p, bool pair, int
     for (int c = 0; c < Vec<T>::W; ++c) v[c] = p[c * up];
   }
 }
-template <typename T, typename TO>
-__device__ __forceinline__ void put_cols(TO* __restrict__ p, bool pair, int up, const T (&v)[Vec<T>::W]) {
-  if (Vec<T>::W == 2 && sizeof(TO) == 4 && pair) {
+template <bool FULL, typename T, typename TO>
+__device__ __forceinline__ void put_cols(TO* __restrict__ p, int up, const T (&v)[Vec<T>::W]) {
+  if (Vec<T>::W == 2 && sizeof(TO) == 4 && FULL) {
     *reinterpret_cast<float2*>(p) = make_float2((float)v[0], (float)v[Vec<T>::W - 1]);
   } else {
     p[0] = (TO)v[0];
-    if (Vec<T>::W == 2 && up) p[1] = (TO)v[Vec<T>::W - 1];
+    if (Vec<T>::W == 2 && (FULL || up)) p[1] = (TO)v[Vec<T>::W - 1];
   }
 }
 
-template <typename T, typename TO, int MODE>
-__global__ void __launch_bounds__(kMaxThreads) k_cols(Axis<T> ax, Cols<T, TO> a) {
+template <typename T, typename TO, int MODE, bool FULL>
+__device__ __forceinline__ void cols(const Axis<T>& ax, const Cols<T, TO>& a, int i0, uint32_t off,
+                                     typename Vec<T>::V* tab, int (*mag)[kMaxWarps]) {
   using V = typename Vec<T>::V;
   constexpr int W = Vec<T>::W;
-  extern __shared__ __align__(16) unsigned char smem[];
-  V* tab = reinterpret_cast<V*>(smem);
-  V* S1 = tab + table_elems(ax) + kPad;
-  V* S2 = S1 + lines_elems(ax, a.n);
-  __shared__ int mag[2][kMaxWarps];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nt = blockDim.x, nw = nt >> 5;
-  const int o = blockIdx.x / a.chunks, i0 = (blockIdx.x - o * a.chunks) * a.n * W;
-  const int im = a.im0 + blockIdx.y, C = ax.C, inner = a.inner;
-  const int nl = min(a.n, (inner - i0 + W - 1) / W);
-  const uint32_t inv_nl = div_magic(nl);
-  const bool pair = (inner & 1) == 0;
-  const size_t off = (size_t)o * C * inner + i0;  // within an image
-  const T* src = a.in + (size_t)im * a.N + off;
+  const int C = ax.C, nl = a.n.n;
+  const uint32_t inner = a.inner;
+  V* S1 = tab + table_elems(ax) + kPad;
+  V* S2 = S1 + lines_elems(ax, nl);
+  const int im = a.im0 + blockIdx.y;
+  // columns past the last repeat it, as rows
+  const auto at_col = [&](int l) { return FULL ? l * W : min(i0 + l * W, a.inner - 1) - i0; };
+  const auto has_up = [&](int l) { return FULL || i0 + l * W + 1 < a.inner ? 1 : 0; };
+  const auto valid = [&](int l) { return FULL || i0 + l * W < a.inner; };
   const V* g = load_table(ax, tab, tid, nt);
   zero_pads(ax, S1, nl, tid, nt);
   if (MODE == kDiv || MODE == kMid) zero_pads(ax, S2, nl, tid, nt);
+  wait_previous();
   typename Vec<T>::M m = 0;
+  const T* src = a.in + (size_t)im * a.N + off;
 #pragma unroll 2
   for (int e = tid; e < nl * (ax.C8 / 2); e += nt) {
-    const int yh = fast_div(e, nl, inv_nl), l = e - yh * nl, y = 2 * yh;
-    const int up = i0 + l * W + 1 < inner ? 1 : 0;
+    const int yh = a.n(e), l = e - yh * nl, y = 2 * yh;
+    const T* s = src + (uint32_t)(y * inner + at_col(l));
     V v[2];
 #pragma unroll
     for (int r = 0; r < 2; ++r) {
       T t[W];
 #pragma unroll
       for (int c = 0; c < W; ++c) t[c] = T(0);
-      if (y + r < C) get_cols<T>(src + (size_t)(y + r) * inner + l * W, pair, up, t);
+      if (FULL || y + r < C) get_cols<FULL>(s + r * inner, has_up(l), t);
       m = Vec<T>::up(m, t);
       v[r] = Vec<T>::make(t);
     }
@@ -578,16 +633,17 @@ __global__ void __launch_bounds__(kMaxThreads) k_cols(Axis<T> ax, Cols<T, TO> a)
   const int xmag = get_mag(mag[0], nw, lane);
   TO* dst = a.out + (size_t)im * a.N + off;
   const auto store = [&](int l, int c0, const V(&acc)[8], const T(&)[1][8][W]) {
-    const int up = i0 + l * W + 1 < inner ? 1 : 0;
+    if (!valid(l)) return;
+    uint32_t i = c0 * inner + l * W;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
+    for (int j = 0; j < 8; ++j, i += inner) {
       T t[W];
       Vec<T>::split(acc[j], t);
-      if (c0 + j < C) put_cols<T, TO>(dst + (size_t)(c0 + j) * inner + l * W, pair, up, t);
+      if (FULL || c0 + j < C) put_cols<FULL, T, TO>(dst + i, has_up(l), t);
     }
   };
   if constexpr (MODE == kOp) {
-    fir_lines<T, 0>(S1, g, ax, nl, inv_nl, xmag, warp, nw, lane, NoExt<T>(), store);
+    fir_lines<T, 0>(S1, g, ax, a.n, xmag, warp, nw, lane, NoExt<T>(), store);
   } else {
     const int pk = im >= a.PK ? im - a.PK : im;
     const bool weights = MODE != kDiv && im >= a.PK;
@@ -598,15 +654,14 @@ __global__ void __launch_bounds__(kMaxThreads) k_cols(Axis<T> ax, Cols<T, TO> a)
     constexpr int kAt = 0, kCb = MODE == kMid ? 1 : 0, kExt = MODE == kMid ? 2 : 1;
     m = 0;
     fir_lines<T, kExt>(
-        S1, g, ax, nl, inv_nl, xmag, warp, nw, lane,
+        S1, g, ax, a.n, xmag, warp, nw, lane,
         [&](int l, int c0, T(&ext)[kExt][8][W]) {
-          const int up = i0 + l * W + 1 < inner ? 1 : 0;
+          uint32_t i = c0 * inner + at_col(l);
 #pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            const size_t i = (size_t)(c0 + j) * inner + l * W;
-            if (c0 + j < C) {
-              if (MODE != kMidLast) get_cols<T>(at + i, pair, up, ext[kAt][j]);
-              if (MODE != kDiv) get_cols<T>(cbr + i, pair, up, ext[kCb][j]);
+          for (int j = 0; j < 8; ++j, i += inner) {
+            if (FULL || c0 + j < C) {
+              if (MODE != kMidLast) get_cols<FULL>(at + i, has_up(l), ext[kAt][j]);
+              if (MODE != kDiv) get_cols<FULL>(cbr + i, has_up(l), ext[kCb][j]);
             } else {
 #pragma unroll
               for (int c = 0; c < W; ++c) ext[kAt][j][c] = ext[kCb][j][c] = T(1);
@@ -614,18 +669,17 @@ __global__ void __launch_bounds__(kMaxThreads) k_cols(Axis<T> ax, Cols<T, TO> a)
           }
         },
         [&](int l, int c0, const V(&acc)[8], const T(&ext)[kExt][8][W]) {
-          const int up = i0 + l * W + 1 < inner ? 1 : 0;
           V nx[8];
+          uint32_t i = c0 * inner + l * W;
 #pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            const size_t i = (size_t)(c0 + j) * inner + l * W;
+          for (int j = 0; j < 8; ++j, i += inner) {
             T c[W], w[W];
             Vec<T>::split(acc[j], c);
 #pragma unroll
             for (int h = 0; h < W; ++h) w[h] = T(0);
-            if (c0 + j < C) {
+            if (FULL || c0 + j < C) {
               if (MODE == kDiv) {
-                if (cbw) put_cols<T, T>(cbw + i, pair, up, c);
+                if (cbw && valid(l)) put_cols<FULL, T, T>(cbw + i, has_up(l), c);
 #pragma unroll
                 for (int h = 0; h < W; ++h) w[h] = ext[kAt][j][h] / c[h];
               } else if (weights) {
@@ -638,7 +692,7 @@ __global__ void __launch_bounds__(kMaxThreads) k_cols(Axis<T> ax, Cols<T, TO> a)
                   qv[h] = c[h] / ext[kCb][j][h];
                   if (MODE == kMid) w[h] = -ext[kAt][j][h] * c[h] / (ext[kCb][j][h] * ext[kCb][j][h]);
                 }
-                put_cols<T, T>(qw + i, pair, up, qv);
+                if (valid(l)) put_cols<FULL, T, T>(qw + i, has_up(l), qv);
               }
               m = Vec<T>::up(m, w);
             }
@@ -650,13 +704,25 @@ __global__ void __launch_bounds__(kMaxThreads) k_cols(Axis<T> ax, Cols<T, TO> a)
     if (MODE == kDiv && a.range && !Vec<T>::finite(m)) a.range[im / a.K] = 1;
     put_mag<T>(mag[1], m, warp, lane);
     __syncthreads();
-    fir_lines<T, 0>(S2, g, ax, nl, inv_nl, get_mag(mag[1], nw, lane), warp, nw, lane, NoExt<T>(), store);
+    fir_lines<T, 0>(S2, g, ax, a.n, get_mag(mag[1], nw, lane), warp, nw, lane, NoExt<T>(), store);
   }
 }
 
-// Loss and its gradient (cpp/loss.h:19-90) over 2048-pixel segments: n the loss
+template <typename T, typename TO, int MODE>
+__global__ void __launch_bounds__(kMaxThreads, 3) k_cols(Axis<T> ax, Cols<T, TO> a) {
+  start_next();
+  extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ int mag[2][kMaxWarps];
+  const int o = blockIdx.x / a.chunks, i0 = (blockIdx.x - o * a.chunks) * a.n.n * Vec<T>::W;
+  const uint32_t off = (uint32_t)o * ax.C * a.inner + i0;  // within an image
+  auto* tab = reinterpret_cast<typename Vec<T>::V*>(smem);
+  const bool full = (ax.C & 7) == 0 && i0 + a.n.n * Vec<T>::W <= a.inner && (Vec<T>::W == 1 || (a.inner & 1) == 0);
+  if (full) cols<T, TO, MODE, true>(ax, a, i0, off, tab, mag);
+  else cols<T, TO, MODE, false>(ax, a, i0, off, tab, mag);
+}
+
+// Loss and its gradient (cpp/loss.h:19-90) over segments of kLossSeg pixels: n the loss
 // gradient, gw = n bary, part the segment's share of the loss.
-constexpr int kLossSeg = 2048;
 template <typename T>
 __global__ void k_loss_seg(const T* __restrict__ bary, const double* __restrict__ obs,
                            const T* __restrict__ wgrad, T* __restrict__ n, T* __restrict__ gw,
@@ -719,23 +785,49 @@ int want_smem(wdl_ctx* ctx, F f, size_t bytes) {
   return WDL_OK;
 }
 
+// A launch of the chain (see start_next).  Overlapped starts pay where they hide a
+// tail (several waves of blocks: images272 8.55 -> 8.30 ms) or a host that issues
+// the launches one by one (the operator: 26.6 -> 20.5 us on volumes); in a
+// replayed graph of small launches they cost 2 us each (dict64 0.87 -> 1.08 ms).
+template <typename... Args, typename... Vals>
+int launch_chained(wdl_ctx* ctx, void (*kernel)(Args...), dim3 grid, int threads, size_t smem, cudaStream_t s,
+                   const Vals&... vals) {
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  const bool waves = (size_t)grid.x * grid.y >= 4 * (size_t)ctx->sm_count;
+  if (!waves) cudaStreamIsCapturing(s, &cap);
+  int rc;
+  if ((rc = want_smem(ctx, kernel, smem))) return rc;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = waves || cap == cudaStreamCaptureStatusNone ? 1 : 0;
+  WDL_CUDA_TRY(ctx, cudaLaunchKernelEx(&cfg, kernel, (Args)vals...));
+  WDL_LAUNCH_CHECK(ctx);
+  return WDL_OK;
+}
+
 template <typename T, typename TO, int MODE>
 int launch_cols(wdl_ctx* ctx, int axis, int outer, int inner, Cols<T, TO> a, size_t nimg, cudaStream_t s) {
   const Axis<T> ax = make_axis<T>(ctx, axis);
-  a.n = cols_per_block(ax.G);
-  const int w = a.n * Vec<T>::W, threads = threads_for(a.n * ax.G);
+  const int nl = cols_per_block(ax.G), w = nl * Vec<T>::W, threads = threads_for(nl * ax.G);
+  a.n = Div::by(nl);
   a.inner = inner;
   a.chunks = (inner + w - 1) / w;
   a.N = ctx->N;
-  const size_t smem = band_smem(ax, MODE == kOp || MODE == kMidLast ? 1 : 2, a.n);
+  const size_t smem = band_smem(ax, MODE == kOp || MODE == kMidLast ? 1 : 2, nl);
   int rc;
-  if ((rc = want_smem(ctx, k_cols<T, TO, MODE>, smem))) return rc;
   const int first = a.im0;
   for (size_t done = 0; done < nimg; done += 65535) {  // gridDim.y is limited to 65535
     const unsigned n = (unsigned)std::min<size_t>(nimg - done, 65535);
     a.im0 = first + (int)done;
-    k_cols<T, TO, MODE><<<dim3((unsigned)(a.chunks * outer), n), threads, smem, s>>>(ax, a);
-    WDL_LAUNCH_CHECK(ctx);
+    if ((rc = launch_chained(ctx, k_cols<T, TO, MODE>, dim3((unsigned)(a.chunks * outer), n), threads, smem, s, ax, a)))
+      return rc;
   }
   return WDL_OK;
 }
@@ -746,12 +838,11 @@ int launch_rows_op(wdl_ctx* ctx, const TI* in, T* out, size_t nimg, cudaStream_t
   const int rows = (int)(ctx->N / ax.C), nl = lines_per_block(1, ax.G, 1), nr = nl * Vec<T>::W;
   const size_t smem = band_smem(ax, 1, nl);
   int rc;
-  if ((rc = want_smem(ctx, k_rows_op<TI, T>, smem))) return rc;
   for (size_t done = 0; done < nimg; done += 65535) {
     const unsigned n = (unsigned)std::min<size_t>(nimg - done, 65535);
-    k_rows_op<TI, T><<<dim3((unsigned)((rows + nr - 1) / nr), n), threads_for(nl * ax.G), smem, s>>>(
-        ax, in ? in + done * ctx->N : nullptr, out + done * ctx->N, rows, nl);
-    WDL_LAUNCH_CHECK(ctx);
+    if ((rc = launch_chained(ctx, k_rows_op<TI, T>, dim3((unsigned)((rows + nr - 1) / nr), n), threads_for(nl * ax.G),
+                             smem, s, ax, in ? in + done * ctx->N : nullptr, out + done * ctx->N, rows, Div::by(nl))))
+      return rc;
   }
   return WDL_OK;
 }
@@ -791,6 +882,9 @@ struct RowsShape {
     n = lines_per_block(K, ax.G, 1);
     nchunk = (rows + n * Vec<T>::W - 1) / (n * Vec<T>::W);
   }
+  // one thread per item or, where there are more, per element of the step between
+  // the passes
+  int threads(int items) const { return threads_for(std::max(items, n * ax.C)); }
   size_t fwd_smem(int K) const { return band_smem(ax, 2, K * n); }
   size_t bwd_smem(int K) const { return band_smem(ax, 2, 2 * K * n) + (size_t)kMaxWarps * K * sizeof(double); }
 };
@@ -798,7 +892,7 @@ struct RowsShape {
 // Every line buffer of a call fits the SM's shared memory.
 template <typename T>
 bool band_fits(const wdl_ctx* ctx, int K) {
-  if (ctx->N >= ((size_t)1 << 31)) return false;
+  if (K > kMaxK || ctx->N * (size_t)(K > 0 ? K : 1) >= ((size_t)1 << 31)) return false;
   for (int a = 0; a < ctx->ndim; ++a) {
     const Axis<T> ax = make_axis<T>(ctx, a);
     if (ax.C > 8192) return false;
@@ -809,6 +903,20 @@ bool band_fits(const wdl_ctx* ctx, int K) {
   }
   return true;
 }
+// Taps of a group of eight outputs over data of a few bits' spread against the
+// dense split-BF16 axis passes of grids above 128 (272 x 240, 8 histograms, K = 4,
+// L = 50): 8.6 against 11.2 ms at gamma 25 (72 taps), 11.4 against 12.5 at 80
+// (120), 12.6 against 12.5 at 120 (144), 14.7 against 13.2 at 200 (176); one
+// histogram 3.9 against 5.7 ms at gamma 100.
+bool band_narrow(const wdl_ctx* ctx) {
+  for (int a = 0; a < ctx->ndim; ++a) {
+    const Axis<float> ax = make_axis<float>(ctx, a);
+    const int r4 = ((int)std::ceil(std::sqrt((double)ax.k1 * (ax.base + 2))) + 3) & ~3;
+    if (std::min(ax.C8, 8 + 2 * std::min(r4, ax.C8)) > 144) return false;
+  }
+  return true;
+}
+
 template bool band_fits<float>(const wdl_ctx*, int);
 template bool band_fits<double>(const wdl_ctx*, int);
 
@@ -843,7 +951,7 @@ template <typename T>
 int band_forward(wdl_ctx* ctx, const BandEval<T>& e, const T* b0, cudaStream_t s) {
   const RowsShape<T> sh(ctx, e.K);
   const size_t N = ctx->N, PK = (size_t)e.P * e.K, PKN = PK * N, PN = (size_t)e.P * N;
-  const unsigned blocks = (unsigned)((size_t)e.P * sh.nchunk), threads = threads_for(e.K * sh.n * sh.ax.G);
+  const unsigned blocks = (unsigned)((size_t)e.P * sh.nchunk), threads = sh.threads(e.K * sh.n * sh.ax.G);
   const size_t smem = sh.fwd_smem(e.K);
   const bool vol = ctx->ndim == 3;
   int rc;
@@ -866,40 +974,48 @@ int band_forward(wdl_ctx* ctx, const BandEval<T>& e, const T* b0, cudaStream_t s
       c.out = e.t2;
       if ((rc = launch_cols<T, T, kDiv>(ctx, 1, 1, ctx->W, c, PK, s))) return rc;
     }
-    T* phi = e.phi ? e.phi + it * PKN : nullptr;
-    T* bary = e.phi ? e.bary + it * PN : it == e.L - 1 ? e.bary : nullptr;
-    T* t1 = it == e.L - 1 ? nullptr : e.t1;
-#define WDL_ROWS_FWD(KT)                                                                            \
-  if ((rc = want_smem(ctx, k_rows_fwd<T, KT>, smem))) return rc;                                    \
-  k_rows_fwd<T, KT><<<blocks, threads, smem, s>>>(sh.ax, e.t2, e.lam64, phi, bary, t1, e.range, e.K, sh.rows, sh.n, \
-                                                  sh.nchunk)
+    FwdRows<T> a{};
+    a.t2 = e.t2;
+    a.lam = e.lam64;
+    a.phi = e.phi ? e.phi + it * PKN : nullptr;
+    a.bary = e.phi ? e.bary + it * PN : it == e.L - 1 ? e.bary : nullptr;
+    a.t1 = it == e.L - 1 ? nullptr : e.t1;
+    a.range = e.range;
+    a.K = e.K;
+    a.rows = sh.rows;
+    a.nchunk = sh.nchunk;
+    a.nv = Div::by(sh.n);
+    a.nl = Div::by(e.K * sh.n);
+    a.C = Div::by(sh.ax.C);
+#define WDL_ROWS_FWD(KT) rc = launch_chained(ctx, k_rows_fwd<T, KT>, dim3(blocks), (int)threads, smem, s, sh.ax, a)
     WDL_BY_K(e.K, WDL_ROWS_FWD)
 #undef WDL_ROWS_FWD
-    WDL_LAUNCH_CHECK(ctx);
+    if (rc) return rc;
   }
   return WDL_OK;
 }
 template int band_forward<float>(wdl_ctx*, const BandEval<float>&, const float*, cudaStream_t);
 template int band_forward<double>(wdl_ctx*, const BandEval<double>&, const double*, cudaStream_t);
 
-// Loss partials and the reverse pass's start n, gw from the last barycenter.
+// Loss partials (loss_parts per histogram) and the reverse pass's start n, gw from
+// the barycenters.
 template <typename T>
-int band_loss(wdl_ctx* ctx, const BandEval<T>& e, const double* obs, const T* wgrad, int loss_type,
-              cudaStream_t s) {
-  const size_t N = ctx->N, PN = (size_t)e.P * N;
-  const T* bary = e.bary + (size_t)(e.L - 1) * PN;
-  for (int done = 0; done < e.P; done += 65535) {
-    const int n = std::min(e.P - done, 65535);
-    const size_t o = (size_t)done * N, seg = (N + kLossSeg - 1) / kLossSeg;
-    k_loss_seg<T><<<dim3((unsigned)seg, (unsigned)n), 256, 0, s>>>(bary + o, obs + o, wgrad ? wgrad + o : nullptr,
-                                                                   e.n + o, e.gw + o, e.lossp + done * seg,
-                                                                   loss_type, N);
+int loss_segments(wdl_ctx* ctx, int P, const T* bary, const double* obs, const T* wgrad, T* n, T* gw, double* part,
+                  int loss_type, cudaStream_t s) {
+  const size_t N = ctx->N, seg = loss_parts(ctx);
+  for (int done = 0; done < P; done += 65535) {
+    const int np = std::min(P - done, 65535);
+    const size_t o = (size_t)done * N;
+    k_loss_seg<T><<<dim3((unsigned)seg, (unsigned)np), 256, 0, s>>>(bary + o, obs + o, wgrad ? wgrad + o : nullptr,
+                                                                    n + o, gw + o, part + done * seg, loss_type, N);
     WDL_LAUNCH_CHECK(ctx);
   }
   return WDL_OK;
 }
-template int band_loss<float>(wdl_ctx*, const BandEval<float>&, const double*, const float*, int, cudaStream_t);
-template int band_loss<double>(wdl_ctx*, const BandEval<double>&, const double*, const double*, int, cudaStream_t);
+template int loss_segments<float>(wdl_ctx*, int, const float*, const double*, const float*, float*, float*, double*,
+                                  int, cudaStream_t);
+template int loss_segments<double>(wdl_ctx*, int, const double*, const double*, const double*, double*, double*,
+                                   double*, int, cudaStream_t);
 
 template <typename T>
 size_t band_dot_parts(const wdl_ctx* ctx, int K) {
@@ -907,7 +1023,6 @@ size_t band_dot_parts(const wdl_ctx* ctx, int K) {
 }
 template size_t band_dot_parts<float>(const wdl_ctx*, int);
 template size_t band_dot_parts<double>(const wdl_ctx*, int);
-size_t band_loss_parts(const wdl_ctx* ctx) { return (ctx->N + kLossSeg - 1) / kLossSeg; }
 
 // Reverse pass: dot (raw weight gradient), gdic (raw atom gradient, summed over
 // the histograms; cleared by the caller with dotp) when e.dict, and with a
@@ -919,7 +1034,7 @@ int band_backward(wdl_ctx* ctx, const BandEval<T>& e, double* loss, cudaStream_t
   const unsigned blocks = (unsigned)((size_t)e.P * sh.nchunk);
   // the same threads with and without the dictionary recursion: the dot
   // products' order of summation depends on them
-  const unsigned threads = threads_for(2 * e.K * sh.n * sh.ax.G);
+  const unsigned threads = sh.threads(2 * e.K * sh.n * sh.ax.G);
   const size_t smem = sh.bwd_smem(e.K);
   const bool vol = ctx->ndim == 3;
   const int im0 = e.dict ? 0 : (int)PK;
@@ -934,7 +1049,9 @@ int band_backward(wdl_ctx* ctx, const BandEval<T>& e, double* loss, cudaStream_t
   a.K = e.K;
   a.P = e.P;
   a.rows = sh.rows;
-  a.nv = sh.n;
+  a.nv = Div::by(sh.n);
+  a.nl = Div::by(e.K * sh.n);
+  a.C = Div::by(sh.ax.C);
   a.nchunk = sh.nchunk;
   a.nblocks = (int)blocks;
   a.dict = e.dict;
@@ -949,17 +1066,12 @@ int band_backward(wdl_ctx* ctx, const BandEval<T>& e, double* loss, cudaStream_t
     a.want_u = step > 1;
     const bool first = step == e.L;
     const unsigned grid = blocks + (first ? 0 : sum_blocks);
-#define WDL_ROWS_BWD(KT)                                                          \
-  if (first) {                                                                    \
-    if ((rc = want_smem(ctx, k_rows_bwd<T, KT, true>, smem))) return rc;          \
-    k_rows_bwd<T, KT, true><<<grid, threads, smem, s>>>(sh.ax, a);                  \
-  } else {                                                                        \
-    if ((rc = want_smem(ctx, k_rows_bwd<T, KT, false>, smem))) return rc;         \
-    k_rows_bwd<T, KT, false><<<grid, threads, smem, s>>>(sh.ax, a);                 \
-  }
+#define WDL_ROWS_BWD(KT)                                                                                        \
+  rc = first ? launch_chained(ctx, k_rows_bwd<T, KT, true>, dim3(grid), (int)threads, smem, s, sh.ax, a)         \
+             : launch_chained(ctx, k_rows_bwd<T, KT, false>, dim3(grid), (int)threads, smem, s, sh.ax, a)
     WDL_BY_K(e.K, WDL_ROWS_BWD)
 #undef WDL_ROWS_BWD
-    WDL_LAUNCH_CHECK(ctx);
+    if (rc) return rc;
     if (step == 1 && !e.dict) break;
     const size_t nimg = step > 1 ? (e.dict ? 2 * PK : PK) : PK;
     Cols<T, T> c{};
@@ -981,11 +1093,12 @@ int band_backward(wdl_ctx* ctx, const BandEval<T>& e, double* loss, cudaStream_t
   }
   if (e.dict) {  // the last round's share
     a.nblocks = 0;
-    k_rows_bwd<T, 0, true><<<grid_for(KN, (int)threads, ctx->sm_count), threads, 0, s>>>(sh.ax, a);
-    WDL_LAUNCH_CHECK(ctx);
+    if ((rc = launch_chained(ctx, k_rows_bwd<T, 0, true>, dim3(grid_for(KN, (int)threads, ctx->sm_count)), (int)threads,
+                             (size_t)0, s, sh.ax, a)))
+      return rc;
   }
   k_band_sums<<<(unsigned)(PK + (loss ? e.P : 0)), 256, 0, s>>>(e.dotp, e.dot, (int)PK, sh.nchunk, e.lossp,
-                                                              loss, (int)band_loss_parts(ctx));
+                                                              loss, (int)loss_parts(ctx));
   WDL_LAUNCH_CHECK(ctx);
   return WDL_OK;
 }

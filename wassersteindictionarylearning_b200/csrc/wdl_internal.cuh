@@ -216,7 +216,7 @@ inline int log_conv_stack<double>(wdl_ctx* ctx, const double* in, double* out, d
 // and t2 ([dictionary | weights][P][K][N]; barycenters one [P][K][N]), c / conv_b
 // of a round q [P][K][N], the loss gradient n and n * bary gw [P][N], the atom
 // gradient gdic [K][N], partial dot products and losses (band_dot_parts per
-// (p, k), band_loss_parts per p), dot [P][K], range [P] (FP32) or null.
+// (p, k), loss_parts per p), dot [P][K], range [P] (FP32) or null.
 template <typename T>
 struct BandEval {
   int P, K, L, dict;
@@ -229,16 +229,21 @@ struct BandEval {
 // Whether the lines of a call fit shared memory (K = 0: the operator alone).
 template <typename T>
 bool band_fits(const wdl_ctx* ctx, int K);
+// Whether the factor is narrow enough for FP32 band sums to beat tensor-core axis passes.
+bool band_narrow(const wdl_ctx* ctx);
 template <typename T>
 size_t band_dot_parts(const wdl_ctx* ctx, int K);
-size_t band_loss_parts(const wdl_ctx* ctx);
 template <typename TI, typename T, typename TO>
 int band_conv(wdl_ctx* ctx, const TI* in, TO* out, T* tmp, T* tmp2, size_t nimg, cudaStream_t s);
 template <typename T>
 int band_forward(wdl_ctx* ctx, const BandEval<T>& e, const T* b0, cudaStream_t s);
+// Loss partials over segments of kLossSeg pixels (of any CUDA-core path) and the
+// reverse pass's start n, gw.
+constexpr size_t kLossSeg = 2048;
+inline size_t loss_parts(const wdl_ctx* ctx) { return (ctx->N + kLossSeg - 1) / kLossSeg; }
 template <typename T>
-int band_loss(wdl_ctx* ctx, const BandEval<T>& e, const double* obs, const T* wgrad, int loss_type,
-              cudaStream_t s);
+int loss_segments(wdl_ctx* ctx, int P, const T* bary, const double* obs, const T* wgrad, T* n, T* gw, double* part,
+                  int loss_type, cudaStream_t s);
 template <typename T>
 int band_backward(wdl_ctx* ctx, const BandEval<T>& e, double* loss, cudaStream_t s);
 
