@@ -9,14 +9,19 @@
 // per-step dot products are resultLa.  Around it runs liblbfgs' algorithm
 // (lbfgs_dev.cuh), as regress_both runs it around evaluate_both.
 //
-// Each problem gets a group of CTAs by its size: 1 (sides <= 32), a cluster of
-// 2 (<= 64), 4 (<= 128) or 16 (above); a cluster splits every pass's rows and
-// every elementwise loop and meets at cluster barriers.  The four classes run
-// as four launches on their own streams, concurrently.  A group never waits
-// on another group, so the launch needs no residency guarantee and has no
-// spin-waits.  The separable log-sum-exp passes follow the CUDA-core
-// operator's (conv_simt.cu): outward taps with the provably negligible tail
-// cut, base-2 FP32, an odd SMEM row stride.
+// Each problem gets a group of CTAs: one, or a cluster of 2 to 16, which splits
+// every pass's rows and every elementwise loop and meets at cluster barriers.
+// A pass covers all K atoms at once (K rows of blocks to share, five barriers
+// per iteration), so that even a 32 x 32 problem can keep a large cluster busy;
+// the cluster's size grows from the class's least (1, 2, 4, 16 for sides up to
+// 32, 64, 128, 512) while the launch keeps within 1.5 CTAs per SM.  12
+// problems of sides 32-96, 4 iterations: 504 -> 140 ms against one atom at a time
+// on the least groups.  The four classes run as four launches on their own
+// streams, concurrently.  A group never waits on another group, so the launch
+// needs no residency guarantee and has no spin-waits.  The separable
+// log-sum-exp passes follow the CUDA-core operator's (conv_simt.cu): outward
+// taps with the provably negligible tail cut, base-2 FP32, an odd SMEM row
+// stride.
 //
 // Why: the uneven workload's problems (sides 32-192, K 3-8, L 25-100) each
 // need ~1000 small launches per evaluation on the operator path, and their
@@ -36,10 +41,11 @@ namespace {
 using namespace lbdev;
 
 constexpr int kLfThreads = 256;
-// CTAs per problem and rows per pass block, by size class; the largest class
-// uses 16-CTA clusters (a non-portable size, falling back to 8) with 8-row
-// blocks, so that a 192-row pass still gives every CTA rows.
+// Least CTAs per problem by size class, the most (a non-portable cluster size,
+// falling back to 8 where the GPU cannot place it), and the rows of a pass block.
 constexpr int kGroups[4] = {1, 2, 4, 16};
+constexpr int kMostGroup = 16;
+constexpr int kLfRows = 16;
 inline int size_class(int W, int H) {
   const int m = W > H ? W : H;
   return m <= 32 ? 0 : m <= 64 ? 1 : m <= 128 ? 2 : 3;
@@ -53,10 +59,10 @@ struct LogFitProblem {
   const float* latoms;   // [K][N] log of the normalised atoms
   const double* obs;     // [N]
   float *tb, *tcb, *tphi;  // tapes (log values): b [L+1][K][N], conv_b [L][K][N], phi [L][K][N]
-  float *t1, *a;         // [N]: transposed intermediate, second operand / result
+  float *t1, *a;         // [K][N]: transposed intermediate, result of an operator
   float *u, *r;          // [K][N]
   float *gw, *blog;      // [N]
-  uint8_t *sw, *ts;      // [K][N] signs, [N] intermediate signs
+  uint8_t *sw, *ts;      // [K][N] signs and intermediate signs
   double* part;          // [group][K + 1] partial sums (dot products, loss)
   double* v;             // L-BFGS vectors (pool_doubles(K))
   double* w64;           // [K] weights of the current trial point
@@ -87,16 +93,23 @@ __device__ double block_sum_d(double v, double* sh) {
   return t;  // in every thread
 }
 
-// One separable log-sum-exp axis pass of one image ([R][C] -> [C][R]), the
-// rows shared among the group: out[c][r] = log sum_k s_k exp(-(c-k)^2/gamma +
-// in[r][k]) (signs optional, in and out sign arrays distinct), as the
-// CUDA-core operator's pass: rows staged with a halo, four neighbouring outputs
-// of a row per thread in one running-maximum pass (log_group.cuh).
-template <bool SIGNED, int G, int LR>
-__device__ void lse_pass(const float* __restrict__ in, float* __restrict__ out, int R, int C, float gamma,
+// What a pass reads at element i of an image: the operand itself, log p - conv_b
+// (the forward second operator's), or c + log p - 2 conv_b (the reverse one's).
+enum { kPlain, kMinus, kMid };
+
+// One separable log-sum-exp axis pass of K images ([R][C] -> [C][R] each, N
+// apart), their row blocks shared among the group: out[c][r] = log sum_k s_k
+// exp(-(c-k)^2/gamma + in[r][k]) (signs optional, in and out sign arrays
+// distinct), as the CUDA-core operator's pass: rows staged with a halo, four
+// neighbouring outputs of a row per thread in one running-maximum pass
+// (log_group.cuh).
+template <bool SIGNED, int PRO, int G>
+__device__ void lse_pass(const float* __restrict__ in, const float* __restrict__ lat, const float* __restrict__ cb,
+                         float* __restrict__ out, int K, int R, int C, float gamma,
                          const uint8_t* __restrict__ in_sign, uint8_t* __restrict__ out_sign, float* sm,
                          int rank) {
   using namespace lse;
+  constexpr int LR = kLfRows;
   const int CP = log_cp(C), SP = log_sp(C);
   float* rows = sm;
   float* lk = rows + LR * CP;
@@ -105,32 +118,39 @@ __device__ void lse_pass(const float* __restrict__ in, float* __restrict__ out, 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int G4 = (C + 3) >> 2;
   const bool full = (C & 3) == 0;
+  const int nb = (R + LR - 1) / LR;  // row blocks of an image
+  const size_t N = (size_t)R * C;
   __syncthreads();
   for (int d = tid; d < C; d += kLfThreads) lk[d] = -float(d) * float(d) / gamma * kLog2e;
-  for (int rb = rank; rb * LR < R; rb += G) {
-    const int r0 = rb * LR, nr = min(LR, R - r0);
+  for (int rb = rank; rb < K * nb; rb += G) {
+    const int k = rb / nb, r0 = (rb - k * nb) * LR, nr = min(LR, R - r0);
+    const size_t base = k * N;
     __syncthreads();
     for (int rr = warp; rr < LR; rr += kLfThreads / 32) {
       float* rw = rows + rr * CP + kHalo;
       uint8_t* sw = sg + rr * SP + kHalo;
-      for (int k = lane; k < kHalo; k += 32) {
-        rw[-kHalo + k] = LogOps<float>::kNone;
-        rw[C + k] = LogOps<float>::kNone;
+      for (int x = lane; x < kHalo; x += 32) {
+        rw[-kHalo + x] = LogOps<float>::kNone;
+        rw[C + x] = LogOps<float>::kNone;
         if (SIGNED) {
-          sw[-kHalo + k] = 1;
-          sw[C + k] = 1;
+          sw[-kHalo + x] = 1;
+          sw[C + x] = 1;
         }
       }
       float vm = kFloorF;
-      for (int k = lane; k < C; k += 32) {
+      for (int x = lane; x < C; x += 32) {
         float v = kFloorF;
         uint8_t sv = 1;
         if (rr < nr) {
-          v = in[(size_t)(r0 + rr) * C + k] * kLog2e;
-          if (SIGNED) sv = in_sign[(size_t)(r0 + rr) * C + k];
+          const size_t i = base + (size_t)(r0 + rr) * C + x;
+          float t = in[i];
+          if (PRO == kMinus) t = lat[i] - t;
+          if (PRO == kMid) t = t + (lat[i] - 2.f * cb[i]);
+          v = t * kLog2e;
+          if (SIGNED) sv = in_sign[i];
         }
-        rw[k] = v;
-        if (SIGNED) sw[k] = sv;
+        rw[x] = v;
+        if (SIGNED) sw[x] = sv;
         vm = fmaxf(vm, v);
       }
       for (int o = 16; o > 0; o >>= 1) vm = fmaxf(vm, __shfl_xor_sync(0xffffffffu, vm, o));
@@ -149,7 +169,7 @@ __device__ void lse_pass(const float* __restrict__ in, float* __restrict__ out, 
       else log_group<float, SIGNED, false>(row, sgn, lk, xmax[rr], c0, C, v, pos);
       const int nv = min(4, C - c0);
       for (int j = 0; j < nv; ++j) {
-        const size_t o = (size_t)(c0 + j) * R + (r0 + rr);
+        const size_t o = base + (size_t)(c0 + j) * R + (r0 + rr);
         out[o] = v[j];
         if (SIGNED) out_sign[o] = pos[j] ? 1 : 0;
       }
@@ -157,17 +177,17 @@ __device__ void lse_pass(const float* __restrict__ in, float* __restrict__ out, 
   }
 }
 
-// The 2-D operator: x pass into t1 (transposed), y pass into out.
-template <bool SIGNED, int G, int LR>
-__device__ void lse_image(const float* in, float* out, const LogFitProblem& p, float gamma, uint8_t* signs,
-                          float* sm, int rank) {
-  lse_pass<SIGNED, G, LR>(in, p.t1, p.H, p.W, gamma, signs, p.ts, sm, rank);
+// The 2-D operator on K images: x pass into t1 (transposed), y pass into out.
+template <bool SIGNED, int PRO, int G>
+__device__ void lse_images(const float* in, const float* cb, float* out, const LogFitProblem& p, float gamma,
+                           uint8_t* signs, float* sm, int rank) {
+  lse_pass<SIGNED, PRO, G>(in, p.latoms, cb, p.t1, p.K, p.H, p.W, gamma, signs, p.ts, sm, rank);
   group_sync<G>();
-  lse_pass<SIGNED, G, LR>(p.t1, out, p.W, p.H, gamma, p.ts, signs, sm, rank);
+  lse_pass<SIGNED, kPlain, G>(p.t1, nullptr, nullptr, out, p.K, p.W, p.H, gamma, p.ts, signs, sm, rank);
   group_sync<G>();
 }
 
-template <int G, int LR>
+template <int G>
 __global__ void __launch_bounds__(kLfThreads)
     log_fit_kernel(const LogFitProblem* __restrict__ probs, int nprob, LbParam prm, float gamma, int max_evals) {
   extern __shared__ float sm[];
@@ -196,12 +216,8 @@ __global__ void __launch_bounds__(kLfThreads)
       const float* bprev = p.tb + (size_t)(it - 1) * KN;
       float* cb = p.tcb + (size_t)(it - 1) * KN;
       float* ph = p.tphi + (size_t)(it - 1) * KN;
-      for (int k = 0; k < K; ++k) {
-        lse_image<false, G, LR>(bprev + k * N, cb + k * N, p, gamma, nullptr, sm, rank);
-        for (size_t j = g0; j < N; j += gstride) p.a[j] = p.latoms[k * N + j] - cb[k * N + j];
-        group_sync<G>();
-        lse_image<false, G, LR>(p.a, ph + k * N, p, gamma, nullptr, sm, rank);
-      }
+      lse_images<false, kPlain, G>(bprev, nullptr, cb, p, gamma, nullptr, sm, rank);
+      lse_images<false, kMinus, G>(cb, nullptr, ph, p, gamma, nullptr, sm, rank);
       float* bnext = p.tb + (size_t)it * KN;
       for (size_t j = g0; j < N; j += gstride) {
         float s = 0.f;
@@ -259,21 +275,17 @@ __global__ void __launch_bounds__(kLfThreads)
       if (s == 1) break;
       const float* cbs = p.tcb + (size_t)(s - 1) * KN;
       const float* bp = p.tb + (size_t)(s - 1) * KN;
-      for (int k = 0; k < K; ++k) {
-        lse_image<true, G, LR>(p.u + k * N, p.a, p, gamma, p.sw + k * N, sm, rank);
-        for (size_t j = g0; j < N; j += gstride)
-          p.u[k * N + j] = p.a[j] + (p.latoms[k * N + j] - 2.f * cbs[k * N + j]);
-        group_sync<G>();
-        lse_image<true, G, LR>(p.u + k * N, p.a, p, gamma, p.sw + k * N, sm, rank);
-        for (size_t j = g0; j < N; j += gstride) {
-          const float ex = expf(p.a[j] + bp[k * N + j]);
-          p.r[k * N + j] = p.sw[k * N + j] ? ex : -ex;
-        }
-        group_sync<G>();
-      }
+      lse_images<true, kPlain, G>(p.u, nullptr, p.a, p, gamma, p.sw, sm, rank);
+      lse_images<true, kMid, G>(p.a, cbs, p.a, p, gamma, p.sw, sm, rank);
       for (size_t j = g0; j < N; j += gstride) {
         float sg = 0.f;
-        for (int k = 0; k < K; ++k) sg -= p.r[k * N + j];
+        for (int k = 0; k < K; ++k) {
+          const size_t i = k * N + j;
+          const float ex = expf(p.a[i] + bp[i]);
+          const float r = p.sw[i] ? ex : -ex;
+          p.r[i] = r;
+          sg -= r;
+        }
         p.gw[j] = sg;
       }
       group_sync<G>();
@@ -306,13 +318,15 @@ size_t lse_smem(int C, int LR) {
   return ((size_t)LR * lse::log_cp(C) + C + LR) * sizeof(float) + (size_t)LR * lse::log_sp(C) + 16;
 }
 
-template <int G, int LR>
+template <int G>
 int launch_log_fit(wdl_ctx* ctx, const LogFitProblem* d_probs, int n, const LbParam& prm, int max_evals,
                    int maxC, cudaStream_t s) {
-  const size_t smem = lse_smem(maxC, LR);
-  auto kern = log_fit_kernel<G, LR>;
-  if (smem > 48 * 1024)
-    WDL_CUDA_TRY(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const size_t smem = lse_smem(maxC, kLfRows);
+  auto kern = log_fit_kernel<G>;
+  // the limit belongs to the kernel: raised to what the largest side takes, so
+  // that a launch from another thread never lowers it
+  WDL_CUDA_TRY(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)lse_smem(512, kLfRows)));
   if (G > 8)
     WDL_CUDA_TRY(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
   if (G == 1) {
@@ -339,20 +353,20 @@ int launch_log_fit(wdl_ctx* ctx, const LogFitProblem* d_probs, int n, const LbPa
 // Whether a 16-CTA cluster of this kernel can be resident at all (a
 // non-portable size; otherwise the class runs on 8-CTA clusters).
 bool big_clusters_fit(size_t smem) {
-  auto kern = log_fit_kernel<16, 8>;
+  auto kern = log_fit_kernel<kMostGroup>;
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
-      (smem > 48 * 1024 &&
-       cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)) {
+      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)lse_smem(512, kLfRows)) != cudaSuccess) {
     cudaGetLastError();
     return false;
   }
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(16);
+  cfg.gridDim = dim3(kMostGroup);
   cfg.blockDim = dim3(kLfThreads);
   cfg.dynamicSmemBytes = smem;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = 16;
+  attr[0].val.clusterDim.x = kMostGroup;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
@@ -402,8 +416,8 @@ extern "C" int wdl_fit_weights_log(wdl_ctx* ctx, const wdl_fit_problem* fp, int 
     b += a256(KN * 4);                  // latoms
     b += a256(N * 8);                   // obs
     b += a256((L + 1) * KN * 4) + 2 * a256(L * KN * 4);  // tapes
-    b += 4 * a256(N * 4) + 2 * a256(KN * 4);             // t1, a, gw, blog, u, r
-    b += a256(KN) + a256(N);            // sw, ts
+    b += 2 * a256(N * 4) + 4 * a256(KN * 4);             // gw, blog, t1, a, u, r
+    b += 2 * a256(KN);                  // sw, ts
     b += a256((size_t)G * (K + 1) * 8) + a256(pool_doubles((int)K) * 8) + a256(K * 8) + a256(K * 4);
     b += a256(sizeof(LbState)) + a256(sizeof(int));
     return b;
@@ -419,7 +433,7 @@ extern "C" int wdl_fit_weights_log(wdl_ctx* ctx, const wdl_fit_problem* fp, int 
     size_t used = a256(sizeof(LogFitProblem) * ent.size()), end = done;
     while (end < ent.size()) {
       const wdl_fit_problem& f = fp[ent[end].q];
-      const size_t b = footprint(f, kGroups[ent[end].cls]);
+      const size_t b = footprint(f, kMostGroup);
       if (end > done && used + b > budget) break;
       ent[end].off = used;
       ent[end].bytes = b;
@@ -450,7 +464,7 @@ extern "C" int wdl_fit_weights_log(wdl_ctx* ctx, const wdl_fit_problem* fp, int 
     for (size_t e : order) {
       const Entry& en = ent[e];
       const wdl_fit_problem& f = fp[en.q];
-      const int G = kGroups[en.cls];
+      const int G = kMostGroup;
       const size_t N = (size_t)f.W * f.H, K = f.K, L = f.L, KN = K * N;
       char* c = base + en.off;
       auto take = [&](size_t bytes) {
@@ -471,14 +485,14 @@ extern "C" int wdl_fit_weights_log(wdl_ctx* ctx, const wdl_fit_problem* fp, int 
       d.tb = reinterpret_cast<float*>(take((L + 1) * KN * 4));
       d.tcb = reinterpret_cast<float*>(take(L * KN * 4));
       d.tphi = reinterpret_cast<float*>(take(L * KN * 4));
-      d.t1 = reinterpret_cast<float*>(take(N * 4));
-      d.a = reinterpret_cast<float*>(take(N * 4));
+      d.t1 = reinterpret_cast<float*>(take(KN * 4));
+      d.a = reinterpret_cast<float*>(take(KN * 4));
       d.gw = reinterpret_cast<float*>(take(N * 4));
       d.blog = reinterpret_cast<float*>(take(N * 4));
       d.u = reinterpret_cast<float*>(take(KN * 4));
       d.r = reinterpret_cast<float*>(take(KN * 4));
       d.sw = reinterpret_cast<uint8_t*>(take(KN));
-      d.ts = reinterpret_cast<uint8_t*>(take(N));
+      d.ts = reinterpret_cast<uint8_t*>(take(KN));
       d.part = reinterpret_cast<double*>(take((size_t)G * (K + 1) * 8));
       d.v = reinterpret_cast<double*>(take(pool_doubles((int)K) * 8));
       d.w64 = reinterpret_cast<double*>(take(K * 8));
@@ -524,6 +538,31 @@ extern "C" int wdl_fit_weights_log(wdl_ctx* ctx, const wdl_fit_problem* fp, int 
     LogFitProblem* d_probs = reinterpret_cast<LogFitProblem*>(base);
     WDL_CUDA_TRY(ctx, cudaMemcpyAsync(d_probs, desc.data(), desc.size() * sizeof(LogFitProblem),
                                       cudaMemcpyHostToDevice, s));
+    // CTAs per problem: from the classes' least, the class with the most work per
+    // CTA doubles its groups while the wave has at most 1.5 CTAs per SM (two fit, but
+    // 16-CTA clusters cannot use every slot)
+    int group[4];
+    double cls_work[4] = {0, 0, 0, 0};  // of a class's heaviest problem
+    long long ctas = 0;
+    for (int cls = 0; cls < 4; ++cls) {
+      group[cls] = kGroups[cls];
+      ctas += (long long)cnt[cls] * group[cls];
+    }
+    for (size_t e = done; e < end; ++e) {
+      const wdl_fit_problem& f = fp[ent[e].q];
+      const double w = (double)f.K * f.L * f.W * f.H * (f.W + f.H);
+      cls_work[ent[e].cls] = std::max(cls_work[ent[e].cls], w);
+    }
+    while (true) {
+      int best = -1;
+      for (int cls = 0; cls < 4; ++cls)
+        if (cnt[cls] && group[cls] < kMostGroup && ctas + (long long)cnt[cls] * group[cls] <= 3LL * ctx->sm_count / 2 &&
+            (best < 0 || cls_work[cls] / group[cls] > cls_work[best] / group[best]))
+          best = cls;
+      if (best < 0) break;
+      ctas += (long long)cnt[best] * group[best];
+      group[best] *= 2;
+    }
     {  // the four classes concurrently, each on a stream of its own
       cudaStream_t cs[4] = {nullptr, nullptr, nullptr, nullptr};
       int first = 0;
@@ -536,17 +575,14 @@ extern "C" int wdl_fit_weights_log(wdl_ctx* ctx, const wdl_fit_problem* fp, int 
           break;
         }
         const LogFitProblem* dp = d_probs + first;
-        switch (cls) {
-          case 0: rc = launch_log_fit<1, 16>(ctx, dp, cnt[0], prm, max_evals, maxC[0], cs[0]); break;
-          case 1: rc = launch_log_fit<2, 16>(ctx, dp, cnt[1], prm, max_evals, maxC[1], cs[1]); break;
-          case 2: rc = launch_log_fit<4, 16>(ctx, dp, cnt[2], prm, max_evals, maxC[2], cs[2]); break;
-          default:
-            if (big_clusters_fit(lse_smem(maxC[3], 8))) {
-              rc = launch_log_fit<16, 8>(ctx, dp, cnt[3], prm, max_evals, maxC[3], cs[3]);
-            } else {
-              rc = launch_log_fit<8, 16>(ctx, dp, cnt[3], prm, max_evals, maxC[3], cs[3]);
-            }
-            break;
+        int G = group[cls];
+        if (G == kMostGroup && !big_clusters_fit(lse_smem(maxC[cls], kLfRows))) G = 8;
+        switch (G) {
+          case 1: rc = launch_log_fit<1>(ctx, dp, cnt[cls], prm, max_evals, maxC[cls], cs[cls]); break;
+          case 2: rc = launch_log_fit<2>(ctx, dp, cnt[cls], prm, max_evals, maxC[cls], cs[cls]); break;
+          case 4: rc = launch_log_fit<4>(ctx, dp, cnt[cls], prm, max_evals, maxC[cls], cs[cls]); break;
+          case 8: rc = launch_log_fit<8>(ctx, dp, cnt[cls], prm, max_evals, maxC[cls], cs[cls]); break;
+          default: rc = launch_log_fit<kMostGroup>(ctx, dp, cnt[cls], prm, max_evals, maxC[cls], cs[cls]); break;
         }
         first += cnt[cls];
       }
