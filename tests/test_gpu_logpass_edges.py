@@ -53,3 +53,25 @@ def test_log_operator_edges(oracle, W, H, gamma, spread, precision):
     else:  # the first pass's signed sums may cancel too; FP32 can flip those
         assert same[cond < 1e2].mean() > 0.99
     k.close()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("gamma,spread", [(0.3, 5.0), (60.0, 5.0), (0.7, 60.0)])
+@pytest.mark.parametrize("W,H", [(1, 1), (1, 5), (2, 3), (5, 9), (7, 8), (31, 33), (37, 130), (300, 6)])
+def test_log_pass_forms_agree(W, H, gamma, spread, precision):
+    """One output per thread and four: the same bits, and the same bits next to
+    other images.  A context's first call times the forms of each pass and ends
+    with the one-output form's result; profiling keeps four outputs per thread."""
+    from wassersteindictionarylearning_b200 import CudaLogSignArrayGaussian2DKernel
+    from wassersteindictionarylearning_b200._lib import lib
+    nv = 3
+    u, signs = _inputs(W, H, nv, spread, seed=W * 10 + H)
+    outs = []
+    for plain in (0, 1):
+        k = CudaLogSignArrayGaussian2DKernel(gamma, W, H, precision=precision)
+        lib().wdl_set_profiling(k.ctx, plain)
+        sg = signs.copy()
+        outs.append((k.log_convolve(u, nv), k.log_convolve_signArray(u, sg, nv), sg))
+        k.close()
+    for a, b in zip(*outs):
+        assert np.array_equal(a, b)

@@ -7,6 +7,7 @@
 // image viewed as [R][C] (C contiguous) is contracted along C with the dense
 // C x C factor and written as [C][R], moving the contracted axis to the front.
 // Applying it once per axis returns the image to its original layout.
+#include <algorithm>
 #include <cstdlib>
 #include <cstring>
 
@@ -287,6 +288,59 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? (SIGNED ? 4 : 5) : 2) lo
   }
 }
 
+// The pass with one output per thread (log_lane): eight rows and four positions
+// per warp, the groups of a row spread over the warps and over gridDim.z blocks.
+// For launches that leave the GPU mostly idle, where a pass takes as long as one
+// thread's chain of taps: a group of four is 8 exponentials a tap on one warp of
+// 32 rows, here 2 on one of 8 rows.  Two 61 x 84 histograms, K = 3, FP64: the unsigned
+// pass 17 us (its best rows per block) -> 6.8 us, the signed pair 20 -> 7.9 us.
+constexpr int kLaneRows = 8;
+template <typename T, bool SIGNED, bool SUB>
+__global__ void __launch_bounds__(256, 2) log_lane_pass_kernel(
+    const T* __restrict__ in, T* __restrict__ out, int R, int C, size_t img_stride, T gamma_t,
+    const uint8_t* __restrict__ in_sign, uint8_t* __restrict__ out_sign,
+    unsigned long long* __restrict__ exps, const T* __restrict__ sub_from, T* __restrict__ sub_out,
+    int sub_k, size_t img0) {
+  constexpr int LR = kLaneRows;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int CP = log_cp(C), SP = log_sp(C);
+  T* rows = reinterpret_cast<T*>(smem_raw);             // laid out as log_axis_pass_kernel's
+  T* lk = rows + LR * CP;
+  T* xmax = lk + C;
+  uint8_t* sg = reinterpret_cast<uint8_t*>(xmax + LR);
+  const int r0 = blockIdx.x * LR;
+  const size_t base = (size_t)blockIdx.y * img_stride;
+  const int nr = min(LR, R - r0);
+  log_stage<T, SIGNED, LR>(in, in_sign, rows, sg, xmax, lk, base, r0, nr, C, CP, SP, gamma_t);
+  __syncthreads();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int rr = lane & 7, q = lane >> 3;
+  const T* row = rows + rr * CP + kHalo;
+  const uint8_t* sgn = sg + rr * SP + kHalo;
+  const T X = xmax[rr];
+  const int G = (C + 3) >> 2;
+  unsigned n_ex = 0;
+  for (int gi = blockIdx.z * 8 + warp; gi < G; gi += 8 * gridDim.z) {  // uniform over the warp
+    const int c0 = 4 * gi, c = c0 + q;
+    T v;
+    bool pos;
+    const int n = log_lane<T, SIGNED>(row, sgn, lk, X, c0, c, C, rr < nr, &v, &pos);
+    if (rr < nr && c < C) {
+      const size_t o = base + (size_t)(c * R + r0 + rr);
+      out[o] = v;
+      if (SIGNED) out_sign[o] = pos ? 1 : 0;
+      if (SUB) sub_out[o] = sub_from[((img0 + blockIdx.y) % (size_t)sub_k) * img_stride + (size_t)(c * R + r0 + rr)] - v;
+      n_ex += (unsigned)n;
+    }
+  }
+  if (exps) {
+    unsigned long long v = n_ex;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if (lane == 0) atomicAdd(exps, v);
+  }
+}
+
 template <typename T>
 size_t log_axis_smem(int LR, int C) {
   return ((size_t)LR * log_cp(C) + C + LR) * sizeof(T) + (size_t)LR * log_sp(C) + 16;
@@ -334,10 +388,41 @@ int log_axis_launch(wdl_ctx* ctx, const T* in, T* out, int R, int C, size_t nimg
   return WDL_OK;
 }
 
+// Blocks of the one-output-per-thread form before its rows are split over gridDim.z.
+inline size_t lane_blocks(int R, size_t nimg) { return (size_t)((R + kLaneRows - 1) / kLaneRows) * nimg; }
+// It is a candidate while those are at most four per SM: from there on the group of four
+// has threads enough, and its taps, weights and stop tests serve four outputs.
+inline bool lane_candidate(const wdl_ctx* ctx, int R, int C, size_t nimg, size_t smem) {
+  return lane_blocks(R, nimg) <= 4 * (size_t)ctx->sm_count && (size_t)R * C < ((size_t)1 << 31) && smem <= 200 * 1024;
+}
+
 template <typename T>
-int log_axis_dispatch(wdl_ctx* ctx, int LR, const T* in, T* out, int R, int C, size_t nimg,
+int log_lane_launch(wdl_ctx* ctx, const T* in, T* out, int R, int C, size_t nimg, size_t img_stride,
+                    const uint8_t* in_sign, uint8_t* out_sign, cudaStream_t s, const T* sub_from,
+                    T* sub_out, int sub_k) {
+  const size_t smem = log_axis_smem<T>(kLaneRows, C), blocks = lane_blocks(R, nimg);
+  unsigned long long* exps = ctx->profiling ? ctx->d_taps : nullptr;
+  // split a row's groups over blocks until each warp has one or the grid is four blocks per SM
+  const int G = (C + 3) / 4;
+  const size_t z = std::max<size_t>(1, std::min<size_t>((G + 7) / 8, 4 * (size_t)ctx->sm_count / blocks));
+  const dim3 grid((unsigned)((R + kLaneRows - 1) / kLaneRows), (unsigned)nimg, (unsigned)z);
+  auto k = in_sign    ? log_lane_pass_kernel<T, true, false>
+           : sub_from ? log_lane_pass_kernel<T, false, true>
+                      : log_lane_pass_kernel<T, false, false>;
+  if (smem > 48 * 1024)
+    WDL_CUDA_TRY(ctx, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+  k<<<grid, 256, smem, s>>>(in, out, R, C, img_stride, T(ctx->gamma), in_sign, out_sign, exps, sub_from, sub_out,
+                            sub_k, 0);
+  WDL_LAUNCH_CHECK(ctx);
+  return WDL_OK;
+}
+
+template <typename T>
+int log_axis_dispatch(wdl_ctx* ctx, int LR, bool lanes, const T* in, T* out, int R, int C, size_t nimg,
                       size_t img_stride, const uint8_t* in_sign, uint8_t* out_sign, cudaStream_t s,
                       const T* sub_from, T* sub_out, int sub_k) {
+  if (lanes)
+    return log_lane_launch<T>(ctx, in, out, R, C, nimg, img_stride, in_sign, out_sign, s, sub_from, sub_out, sub_k);
   // choice: rows per block
   switch (LR) {
     case 8:
@@ -353,7 +438,8 @@ int log_axis_dispatch(wdl_ctx* ctx, int LR, const T* in, T* out, int R, int C, s
 }
 
 // Autotuner: the first call of a shape (rows, row length, image count, type,
-// signed) outside a graph capture runs every candidate rows-per-block on the
+// signed) outside a graph capture runs every candidate (rows per block, and the
+// one-output-per-thread form where the grid is small) on the
 // call's own data (once untimed, once timed with CUDA events on the call's
 // stream) and keeps the fastest for later calls of that shape.  WDL_AUTOTUNE=0
 // keeps the default.
@@ -364,31 +450,34 @@ int log_axis_pass(wdl_ctx* ctx, const T* in, T* out, int R, int C, size_t nimg, 
   const long long key[6] = {1, R, C, (long long)nimg, (long long)sizeof(T), in_sign ? 1 : 0};
   for (const auto& e : ctx->tuned)
     if (!std::memcmp(e.key, key, sizeof(key)))
-      return log_axis_dispatch<T>(ctx, e.choice, in, out, R, C, nimg, img_stride, in_sign, out_sign, s, sub_from, sub_out, sub_k);
+      return log_axis_dispatch<T>(ctx, e.choice, e.lanes, in, out, R, C, nimg, img_stride, in_sign, out_sign, s, sub_from, sub_out, sub_k);
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   cudaStreamIsCapturing(s, &cap);
   if (!autotune_enabled() || !ctx->autotune || cap != cudaStreamCaptureStatusNone || ctx->profiling)
-    return log_axis_dispatch<T>(ctx, kLogRowsDefault, in, out, R, C, nimg, img_stride, in_sign, out_sign, s, sub_from, sub_out, sub_k);
-  const int cand[3] = {8, 16, 32};
+    return log_axis_dispatch<T>(ctx, kLogRowsDefault, false, in, out, R, C, nimg, img_stride, in_sign, out_sign, s, sub_from, sub_out, sub_k);
+  const struct { int rows; bool lanes; } cand[4] = {{8, false}, {16, false}, {32, false}, {kLaneRows, true}};
   int best = kLogRowsDefault;
+  bool best_lanes = false;
   float best_ms = 1e30f;
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   WDL_CUDA_TRY(ctx, cudaEventCreate(&e0));
   WDL_CUDA_TRY(ctx, cudaEventCreate(&e1));
   int rc = WDL_OK;
-  for (int c : cand) {
-    if (log_axis_smem<T>(c, C) > 200 * 1024) continue;
+  for (const auto& c : cand) {
+    if (log_axis_smem<T>(c.rows, C) > 200 * 1024) continue;
+    if (c.lanes && !lane_candidate(ctx, R, C, nimg, log_axis_smem<T>(c.rows, C))) continue;
     // an untimed run first: the first launch of a variant also loads it
-    if ((rc = log_axis_dispatch<T>(ctx, c, in, out, R, C, nimg, img_stride, in_sign, out_sign, s, sub_from, sub_out, sub_k))) break;
+    if ((rc = log_axis_dispatch<T>(ctx, c.rows, c.lanes, in, out, R, C, nimg, img_stride, in_sign, out_sign, s, sub_from, sub_out, sub_k))) break;
     cudaEventRecord(e0, s);
-    if ((rc = log_axis_dispatch<T>(ctx, c, in, out, R, C, nimg, img_stride, in_sign, out_sign, s, sub_from, sub_out, sub_k))) break;
+    if ((rc = log_axis_dispatch<T>(ctx, c.rows, c.lanes, in, out, R, C, nimg, img_stride, in_sign, out_sign, s, sub_from, sub_out, sub_k))) break;
     cudaEventRecord(e1, s);
     cudaEventSynchronize(e1);
     float ms = 0;
     cudaEventElapsedTime(&ms, e0, e1);
     if (ms < best_ms) {
       best_ms = ms;
-      best = c;
+      best = c.rows;
+      best_lanes = c.lanes;
     }
   }
   cudaEventDestroy(e0);
@@ -397,6 +486,7 @@ int log_axis_pass(wdl_ctx* ctx, const T* in, T* out, int R, int C, size_t nimg, 
   wdl_ctx::TuneEntry t;
   std::memcpy(t.key, key, sizeof(key));
   t.choice = best;
+  t.lanes = best_lanes;
   t.ms = best_ms;
   ctx->tuned.push_back(t);
   // the candidates computed identical outputs; the last one's stands

@@ -271,6 +271,75 @@ __device__ __forceinline__ int log_group(const T* __restrict__ row, const uint8_
   return 3 + 2 * (d - 2);
 }
 
+// One output c of the group at c0 (c = c0..c0+3) per lane, the four outputs of a
+// group on the lanes q of equal lane % 8: the same operations on every
+// output, in the same order, under the same group-wide conditions (maxima
+// shared by shuffles), so the same bits as log_group.  go: the lane's row
+// exists; c < C holds for the outputs that count.  All 32 lanes call it with one c0.
+template <typename T, bool SIGNED>
+__device__ __forceinline__ int log_lane(const T* __restrict__ row, const uint8_t* __restrict__ sgn,
+                                        const T* __restrict__ lk, T X, int c0, int c, int C, bool go, T* v,
+                                        bool* pos) {
+  using Op = LogOps<T>;
+  const bool valid = c < C;
+  const T l1 = C > 1 ? lk[1] : Op::kNone;
+  const T cx = row[c], lx = row[c - 1], rx = row[c + 1];
+  T m = vmax(vmax(cx, Op::kFloor), vmax(lx, rx) + l1);
+  const T lm1 = l1 - m;
+  T s;
+  if (SIGNED) {
+    s = sign_of<T>(sgn[c]) * Op::ex(cx - m);
+    s += sign_of<T>(sgn[c - 1]) * Op::ex(lx + lm1);
+    s += sign_of<T>(sgn[c + 1]) * Op::ex(rx + lm1);
+  } else {
+    s = Op::ex(cx - m);
+    s += Op::ex(lx + lm1);
+    s += Op::ex(rx + lm1);
+  }
+  const auto group_min = [&]() {
+    T mn = valid ? m : T(__builtin_huge_val());
+    mn = vmin(mn, __shfl_xor_sync(0xffffffffu, mn, 8));
+    return vmin(mn, __shfl_xor_sync(0xffffffffu, mn, 16));
+  };
+  T mmin = group_min();
+  const int dend = max(min(c0 + 3, C - 1), C - 1 - c0);
+  int d = 2, steps = 0;
+  for (; d <= dend; ++d) {
+    const T l = lk[d];
+    const T bound = l + X;
+    if (bound < mmin - Op::kTail) go = false;
+    if (!__any_sync(0xffffffffu, go)) break;
+    // taps beyond the row: the halo's nearest
+    const int pl = max(c - d, -1), pr = min(c + d, C);
+    const T lm = l - m;
+    T a = row[pl] + lm, b = row[pr] + lm;
+    bool up = false;
+    if (go && bound > mmin) {
+      const T t = vmax(a, b);
+      if (t > T(0)) {
+        s *= Op::ex(-t);
+        m += t;
+        a -= t;
+        b -= t;
+        up = true;
+      }
+    }
+    if (__any_sync(0xffffffffu, up)) mmin = group_min();
+    if (go) {
+      if (SIGNED) {
+        s += sign_of<T>(sgn[pl]) * Op::ex(a);
+        s += sign_of<T>(sgn[pr]) * Op::ex(b);
+      } else {
+        s += Op::ex(a);
+        s += Op::ex(b);
+      }
+      ++steps;
+    }
+  }
+  *pos = SIGNED ? s >= T(0) : true;
+  *v = (Op::lg(SIGNED ? fabs(s) : s) + m) * Op::kUnscale;
+  return 3 + 2 * steps;
+}
 
 // SMEM row strides: values C + 2 kHalo + 1 (odd), sign bytes C + 2 kHalo + 4.
 __host__ __device__ constexpr int log_cp(int C) { return C + 2 * kHalo + 1; }

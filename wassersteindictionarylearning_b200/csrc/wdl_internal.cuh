@@ -119,6 +119,7 @@ struct wdl_ctx {
   struct TuneEntry {
     long long key[6];
     int choice = 0;
+    bool lanes = false;  // log domain: one output per thread (conv_simt.cu)
     float ms = 0;
   };
   std::vector<TuneEntry> tuned;
