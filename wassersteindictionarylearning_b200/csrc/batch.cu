@@ -7,9 +7,10 @@
 // gamma (G[i][j] = g(|i-j|)).  Inputs of all problems are staged in one upload,
 // normalised (Problem::normalize_values, cpp/inverseWasserstein.h:53-74) by one
 // table-driven kernel; the kernel's work items come from a host-built table
-// ordered by round (iteration or reverse step) so that every problem's
-// dependency chain advances in parallel; outputs are gathered into one region
-// and copied back with one transfer.
+// ordered by the share of its rounds (iterations and reverse steps) that a problem has
+// behind it, so that the dependency chains advance in parallel and end together;
+// outputs are gathered into one region and copied back with one transfer.
+#include <algorithm>
 #include <cstring>
 #include <vector>
 
@@ -25,23 +26,29 @@ struct RowJob {          // normalise one row in FP64 and cast it to FP32
   int len;
 };
 
-__global__ void k_rows(const RowJob* __restrict__ jobs, int njobs) {
-  __shared__ double sh[32];
+// A block per row, 1024 threads: a few tens of rows of up to 128 x 128 values leave
+// each SM one row, whose sums are a chain of loads (191 rows: 11 us).
+constexpr int kRowThreads = 1024;
+__global__ void __launch_bounds__(kRowThreads) k_rows(const RowJob* __restrict__ jobs, int njobs) {
+  __shared__ double sh[33];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   for (int jb = blockIdx.x; jb < njobs; jb += gridDim.x) {
     const RowJob j = jobs[jb];
     double s = 0;
-    for (int i = threadIdx.x; i < j.len; i += blockDim.x) s += j.src[i];
+#pragma unroll 4
+    for (int i = threadIdx.x; i < j.len; i += kRowThreads) s += j.src[i];
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = s;
+    if (lane == 0) sh[warp] = s;
     __syncthreads();
-    if (threadIdx.x == 0) {
-      double t = 0;
-      for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += sh[w];
-      sh[31] = t;
+    if (warp == 0) {
+      double t = sh[lane];
+      for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+      if (lane == 0) sh[32] = t;
     }
     __syncthreads();
-    const double tot = sh[31];
-    for (int i = threadIdx.x; i < j.len; i += blockDim.x) {
+    const double tot = sh[32];
+#pragma unroll 4
+    for (int i = threadIdx.x; i < j.len; i += kRowThreads) {
       const double v = j.src[i] / tot;
       if (j.dst64) j.dst64[i] = v;
       j.dst32[i] = (float)v;
@@ -58,10 +65,13 @@ struct OutJob {  // gather an output: 0 = exp(acc), 1 = sum over P of gdic, 2 = 
   size_t len;     // elements of the output
 };
 
+// gridDim.y blocks share a job: an atom gradient of 8 x 128 x 128 is 512 rounds of
+// loads for one block (47 jobs in 32 blocks each: 18 us).
+constexpr unsigned kOutSplit = 32;
 __global__ void k_outputs(const OutJob* __restrict__ jobs, int njobs) {
   for (int jb = blockIdx.x; jb < njobs; jb += gridDim.x) {
     const OutJob j = jobs[jb];
-    for (size_t i = threadIdx.x; i < j.len; i += blockDim.x) {
+    for (size_t i = (size_t)blockIdx.y * blockDim.x + threadIdx.x; i < j.len; i += (size_t)gridDim.y * blockDim.x) {
       if (j.kind == 0) {
         j.dst[i] = (double)expf(j.src[i]);
       } else if (j.kind == 1) {
@@ -260,7 +270,7 @@ int batch_prepare(wdl_ctx* ctx, const wdl_problem* pb, int nprob, size_t extra_b
   if (!outs.empty())
     WDL_CUDA_TRY(ctx, cudaMemcpyAsync(base + bp.outj_off, outs.data(), outs.size() * sizeof(OutJob), cudaMemcpyHostToDevice, s));
   WDL_CUDA_TRY(ctx, cudaMemcpyAsync(base + bp.probs, bp.prs.data(), bp.prs.size() * sizeof(SkProblem), cudaMemcpyHostToDevice, s));
-  k_rows<<<grid_for(rows.size(), 1, ctx->sm_count, 4), 256, 0, s>>>(reinterpret_cast<RowJob*>(base + bp.rows_off), (int)rows.size());
+  k_rows<<<grid_for(rows.size(), 1, ctx->sm_count, 4), kRowThreads, 0, s>>>(reinterpret_cast<RowJob*>(base + bp.rows_off), (int)rows.size());
   WDL_LAUNCH_CHECK(ctx);
   // the error word is cleared here once; every launch clears only the counter
   WDL_CUDA_TRY(ctx, cudaMemsetAsync(bp.sync, 0, 2 * sizeof(int), s));
@@ -269,29 +279,41 @@ int batch_prepare(wdl_ctx* ctx, const wdl_problem* pb, int nprob, size_t extra_b
   return WDL_OK;
 }
 
+// Items are claimed in table order, and an item waits only on earlier rounds of its
+// own problem.  The rounds of all problems are merged in proportion to their
+// number, so that every problem ends at the same time: merged round by round,
+// the short problems crowd the first rounds and the longest one's last rounds run
+// alone, bound by one chain's latency (with the two kernels around the launch: 24 uneven
+// problems 7.03 -> 6.74 ms, 32 of them 6.0 -> 5.64, 12 of them 2.60 -> 2.55).
 void batch_items(const BatchPlan& bp, const std::vector<uint8_t>* active, std::vector<int4>& items) {
   items.clear();
   std::vector<size_t> first(bp.nprob + 1, 0);
-  int rounds_max = 0;
+  struct Round {
+    double at;  // the round's middle, as a fraction of its problem's rounds
+    int q, r;
+  };
+  std::vector<Round> order;
   for (int q = 0; q < bp.nprob; ++q) {
     first[q + 1] = first[q] + bp.prs[q].P;
     const int rounds = bp.prs[q].fwd_only ? bp.prs[q].L : 2 * bp.prs[q].L;
-    if (rounds > rounds_max) rounds_max = rounds;
+    for (int r = 0; r < rounds; ++r) order.push_back({(r + 0.5) / rounds, q, r});
   }
-  for (int r = 0; r < rounds_max; ++r) {
-    for (int q = 0; q < bp.nprob; ++q) {
-      const SkProblem& pr = bp.prs[q];
-      const int PK = pr.P * pr.K;
-      if (r < pr.L) {
-        for (int pk = 0; pk < PK; ++pk)
-          if (!active || (*active)[first[q] + pk / pr.K]) items.push_back(make_int4(q, 0, r + 1, pk));
-      } else if (!pr.fwd_only && r < 2 * pr.L) {
-        const int sstep = 2 * pr.L - r;
-        for (int pk = 0; pk < PK; ++pk) {
-          if (active && !(*active)[first[q] + pk / pr.K]) continue;
-          if (pr.need_dic) items.push_back(make_int4(q, 1, sstep, pk));
-          items.push_back(make_int4(q, 2, sstep, pk));
-        }
+  std::sort(order.begin(), order.end(), [](const Round& a, const Round& b) {
+    return a.at != b.at ? a.at < b.at : a.q != b.q ? a.q < b.q : a.r < b.r;
+  });
+  for (const Round& o : order) {
+    const int q = o.q, r = o.r;
+    const SkProblem& pr = bp.prs[q];
+    const int PK = pr.P * pr.K;
+    if (r < pr.L) {
+      for (int pk = 0; pk < PK; ++pk)
+        if (!active || (*active)[first[q] + pk / pr.K]) items.push_back(make_int4(q, 0, r + 1, pk));
+    } else {
+      const int sstep = 2 * pr.L - r;
+      for (int pk = 0; pk < PK; ++pk) {
+        if (active && !(*active)[first[q] + pk / pr.K]) continue;
+        if (pr.need_dic) items.push_back(make_int4(q, 1, sstep, pk));
+        items.push_back(make_int4(q, 2, sstep, pk));
       }
     }
   }
@@ -340,7 +362,7 @@ extern "C" int wdl_batch_run(wdl_ctx* ctx, const wdl_problem* pb, int nprob) {
   if ((rc = batch_launch(ctx, bp, items.size(), s))) return rc;
   ctx->fused_sync = bp.sync;
   if (bp.n_outjobs) {
-    k_outputs<<<grid_for(bp.n_outjobs, 1, ctx->sm_count, 4), 256, 0, s>>>(reinterpret_cast<OutJob*>(base + bp.outj_off), (int)bp.n_outjobs);
+    k_outputs<<<dim3((unsigned)grid_for(bp.n_outjobs, 1, ctx->sm_count, 4), kOutSplit), 256, 0, s>>>(reinterpret_cast<OutJob*>(base + bp.outj_off), (int)bp.n_outjobs);
     WDL_LAUNCH_CHECK(ctx);
   }
   // ---- results: one download, scattered on the host --------------------------------
