@@ -4,8 +4,8 @@
 //
 // The context's factor matrix serves every problem: the Gibbs factor of a side
 // n is the leading n x n block of the factor of any larger side with the same
-// gamma (G[i][j] = g(|i-j|)).  Inputs of all problems are staged in one upload,
-// normalised (Problem::normalize_values, cpp/inverseWasserstein.h:53-74) by one
+// gamma (G[i][j] = g(|i-j|)).  Images go up by a copy each, straight from the
+// caller's arrays, the weights of all problems in one; they are normalised (Problem::normalize_values, cpp/inverseWasserstein.h:53-74) by one
 // table-driven kernel; the kernel's work items come from a host-built table
 // ordered by the share of its rounds (iterations and reverse steps) that a problem has
 // behind it, so that the dependency chains advance in parallel and end together;
@@ -167,16 +167,16 @@ int batch_prepare(wdl_ctx* ctx, const wdl_problem* pb, int nprob, size_t extra_b
       o.phi = c.take<float>(slots * P * K * N);
       o.sync = c.take<int>(5 * P);
     }
-    bp.in_b = c.mark();  // inputs: one upload
-    for (int q = 0; q < nprob; ++q) {
+    bp.in_b = c.mark();  // weights: one upload
+    for (int q = 0; q < nprob; ++q) bp.buf[q].in_w = c.take<double>((size_t)pb[q].P * pb[q].K);
+    bp.in_e = c.mark();
+    for (int q = 0; q < nprob; ++q) {  // images: a copy each
       const wdl_problem& w = pb[q];
       const size_t N = (size_t)w.W * w.H;
       bp.buf[q].in_atoms = c.take<double>((size_t)w.K * N);
-      bp.buf[q].in_w = c.take<double>((size_t)w.P * w.K);
       bp.buf[q].obs = w.mode == WDL_MODE_BARYCENTER ? nullptr : c.take<double>((size_t)w.P * N);
     }
-    bp.in_e = c.mark();
-    bp.out_b = bp.in_e;  // outputs: one download
+    bp.out_b = c.mark();  // outputs: one download
     for (int q = 0; q < nprob; ++q) {
       const wdl_problem& w = pb[q];
       const size_t N = (size_t)w.W * w.H;
@@ -229,9 +229,10 @@ int batch_prepare(wdl_ctx* ctx, const wdl_problem* pb, int nprob, size_t extra_b
     const wdl_problem& w = pb[q];
     const size_t N = (size_t)w.W * w.H;
     BatchBuf& o = bp.buf[q];
-    std::memcpy(h_in.data() + ((char*)o.in_atoms - base - bp.in_b), w.atoms, (size_t)w.K * N * 8);
+    WDL_CUDA_TRY(ctx, cudaMemcpyAsync(o.in_atoms, w.atoms, (size_t)w.K * N * 8, cudaMemcpyHostToDevice, s));
     std::memcpy(h_in.data() + ((char*)o.in_w - base - bp.in_b), w.weights, (size_t)w.P * w.K * 8);
-    if (o.obs) std::memcpy(h_in.data() + ((char*)o.obs - base - bp.in_b), w.observed, (size_t)w.P * N * 8);
+    if (o.obs)
+      WDL_CUDA_TRY(ctx, cudaMemcpyAsync(o.obs, w.observed, (size_t)w.P * N * 8, cudaMemcpyHostToDevice, s));
     for (int k = 0; k < w.K; ++k) rows.push_back({o.in_atoms + k * N, o.atoms64 + k * N, o.atoms + k * N, (int)N});
     for (int p = 0; p < w.P; ++p) rows.push_back({o.in_w + (size_t)p * w.K, o.lam64 + (size_t)p * w.K, o.lam + (size_t)p * w.K, w.K});
     SkProblem& pr = bp.prs[q];
