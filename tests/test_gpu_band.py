@@ -125,3 +125,24 @@ def test_evaluation_edges(oracle, W, H, D, P, K, L, gamma, precision):
     assert rel(g[P * K:], g_ref[P * K:]) < tol
     scale = oracle.weight_gradient_scale(W, H, D, gamma, P, K, L, 2, cfg["scale_dic"], x, obs)
     assert rel_scaled(g[: P * K], g_ref[: P * K], scale) < tol
+
+
+@pytest.mark.parametrize("precision", ["fp32", "fp64"])
+def test_profile_counts_the_applications(precision):
+    """wdl_conv_profile of an evaluation, in operator applications per atom and histogram:
+    2 per iteration; in the reverse pass 2 per round and recursion, but 1 for the
+    dictionary and none for the weights in the last round."""
+    import ctypes as C
+    from wassersteindictionarylearning_b200 import Problem, WassersteinRegression
+    from wassersteindictionarylearning_b200._lib import lib
+    from wassersteindictionarylearning_b200.synthetic import make_problem, to_variables
+    P, K, L = 2, 3, 4
+    cfg, obs, atoms, w = make_problem(None, seed=1, P=P, W=24, H=17, K=K, L=L, gamma=2.0, loss=2)
+    k = _kernel(24, 17, 1, 2.0, precision)
+    lib().wdl_set_profiling(k.ctx, 1)
+    reg = WassersteinRegression(Problem(np.ones((K, 24 * 17)), obs, k, None, P), L, 2, cfg["scale_dic"])
+    reg.evaluate_both(to_variables(w, atoms, cfg["scale_dic"]))
+    ms, n, apps = C.c_double(), C.c_longlong(), C.c_double()
+    lib().wdl_conv_profile(k.ctx, C.byref(ms), C.byref(n), C.byref(apps))
+    k.close()
+    assert ms.value > 0 and n.value > 0 and apps.value == (2 * L + (2 * L - 1) + 2 * (L - 1)) * P * K

@@ -872,6 +872,27 @@ int plane_cols(wdl_ctx* ctx, const T* in, TO* out, size_t nimg, int im0, cudaStr
 
 }  // namespace
 
+// wdl_conv_profile of a pass over the iterations: the operator is fused with the steps
+// between its applications, so the whole pass counts as one launch of `apps`
+// applications, as the fused tensor-core kernel's does.
+struct PassTimer {
+  wdl_ctx* ctx;
+  cudaStream_t s;
+  PassTimer(wdl_ctx* c, cudaStream_t st) : ctx(c), s(st) {
+    if (ctx->profiling) cudaEventRecord(ctx->ev_a, s);
+  }
+  void done(double apps) {
+    if (!ctx->profiling) return;
+    cudaEventRecord(ctx->ev_b, s);
+    cudaEventSynchronize(ctx->ev_b);
+    float ms = 0;
+    cudaEventElapsedTime(&ms, ctx->ev_a, ctx->ev_b);
+    ctx->conv_ms += ms;
+    ctx->conv_launches += 1;
+    ctx->conv_images += apps;
+  }
+};
+
 // The shape of a rows launch.
 template <typename T>
 struct RowsShape {
@@ -955,6 +976,7 @@ int band_forward(wdl_ctx* ctx, const BandEval<T>& e, const T* b0, cudaStream_t s
   const size_t smem = sh.fwd_smem(e.K);
   const bool vol = ctx->ndim == 3;
   int rc;
+  PassTimer timer(ctx, s);
   if ((rc = launch_rows_op<T, T>(ctx, b0, e.t1, PK, s))) return rc;
   for (int it = 0; it < e.L; ++it) {
     Cols<T, T> c{};
@@ -992,6 +1014,7 @@ int band_forward(wdl_ctx* ctx, const BandEval<T>& e, const T* b0, cudaStream_t s
 #undef WDL_ROWS_FWD
     if (rc) return rc;
   }
+  timer.done(2.0 * e.L * PK);
   return WDL_OK;
 }
 template int band_forward<float>(wdl_ctx*, const BandEval<float>&, const float*, cudaStream_t);
@@ -1039,6 +1062,7 @@ int band_backward(wdl_ctx* ctx, const BandEval<T>& e, double* loss, cudaStream_t
   const bool vol = ctx->ndim == 3;
   const int im0 = e.dict ? 0 : (int)PK;
   int rc;
+  PassTimer timer(ctx, s);
   BwdRows<T> a{};
   a.t2 = e.t2;
   a.n = e.n;
@@ -1100,6 +1124,7 @@ int band_backward(wdl_ctx* ctx, const BandEval<T>& e, double* loss, cudaStream_t
   k_band_sums<<<(unsigned)(PK + (loss ? e.P : 0)), 256, 0, s>>>(e.dotp, e.dot, (int)PK, sh.nchunk, e.lossp,
                                                               loss, (int)loss_parts(ctx));
   WDL_LAUNCH_CHECK(ctx);
+  timer.done(((e.dict ? 2.0 * e.L - 1 : 0.0) + 2.0 * (e.L - 1)) * PK);
   return WDL_OK;
 }
 template int band_backward<float>(wdl_ctx*, const BandEval<float>&, double*, cudaStream_t);
