@@ -14,17 +14,20 @@ namespace wdl {
 // only log(m), which is small, comes from logf.  Used where FP32 logarithms are
 // summed in FP64 over a whole grid (weight-gradient dot products, the weighted
 // geometric mean), so that the sums keep FP32-level relative accuracy.
+// A saturated x = inf stays inf: callers find overflows by it.
 __device__ __forceinline__ double log_f32_precise(float x) {
-  if (x < 1.17549435e-38f) {  // subnormal: scaled to a normal number first
+  const int i = __float_as_int(x);
+  if ((unsigned)(i - 0x00800000) >= 0x7f000000u) {  // not a positive normal number
     int e;
-    float m = frexpf(x, &e);  // x = m * 2^e, m in [0.5, 1)
+    float m = frexpf(x, &e);  // subnormal: x = m * 2^e, m in [0.5, 1)
+    if (!(m < INFINITY)) return (double)m;
     if (m < 0.70710678f) {
       m *= 2.0f;
       e -= 1;
     }
     return (double)e * 0.6931471805599453 + (double)logf(m);
   }
-  const int i = __float_as_int(x), e = (i - 0x3f3504f3) >> 23;  // sqrt(1/2) = 0x3f3504f3
+  const int e = (i - 0x3f3504f3) >> 23;  // sqrt(1/2) = 0x3f3504f3
   const float m = __int_as_float(i - (int)((unsigned)e << 23));
   return (double)e * 0.6931471805599453 + (double)logf(m);
 }
