@@ -777,10 +777,11 @@ __global__ void k_band_sums(const double* __restrict__ dotp, double* __restrict_
 
 // The limit is raised to the most any call takes: it belongs to the kernel, not to
 // the launch, and a smaller value set by another thread in between would refuse
-// this one's.
+// this one's.  48 KB without it hold the kernel's static arrays too.
+constexpr size_t kSmemStatic = 1024;  // at least every kernel's: magnitudes, kMaxK weights
 template <typename F>
 int want_smem(wdl_ctx* ctx, F f, size_t bytes) {
-  if (bytes > 48 * 1024)
+  if (bytes + kSmemStatic > 48 * 1024)
     WDL_CUDA_TRY(ctx, cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMost));
   return WDL_OK;
 }
