@@ -100,7 +100,7 @@ struct Axis {
   int most;      // FP64: largest exponent difference at which EPSILON X stays negligible
   float k1;      // gamma ln 2
   int ext;       // the table in SMEM holds |d| < ext (and d = -ext)
-  int lim[4];    // largest exponent differences served by radii 4, 8, 12, 16
+  int lim[4];    // largest exponent differences served by radii 4, 8, 12, 16 (FP32: any, from the reach on)
 };
 
 // The pitch is an odd number of 16-byte units, so that eight neighbouring

@@ -70,10 +70,13 @@ Axis<T> make_axis(const wdl_ctx* ctx, int axis) {
   ax.most = 830 - ax.base;  // EPSILON = 1e-250 > 2^-831
   ax.k1 = (float)std::min(ctx->gamma * 0.6931471805599453, 1e30);
   // FP64 lines may need every entry (exact zeros), FP32 ones none past the reach
-  ax.ext = sizeof(T) == 8 ? ax.C8 : std::min(ax.C8, ((ax.reach + 3) & ~3) + 8);
+  ax.ext = sizeof(T) == 8 ? ax.C8 : std::min(ax.C8, ((std::max(ax.reach, 1) + 3) & ~3) + 8);
   for (int i = 0; i < 4; ++i) {
     const double r = 4.0 * (i + 1), d = std::floor(r * r / std::max((double)ax.k1, 1e-30)) - ax.base;
     ax.lim[i] = (int)std::min(std::max(d, -1.0), sizeof(T) == 8 ? (double)ax.most : 1e6);
+    // the FP32 factor is zero past its reach: a radius that covers it serves every
+    // difference, and none beyond it is taken (the table holds no more)
+    if (sizeof(T) == 4 && 4 * (i + 1) >= ax.reach) ax.lim[i] = 1000000;
   }
   return ax;
 }
