@@ -13,10 +13,11 @@
 // (kTail = 40 bits for FP32, 60 for FP64: 2^-16 and 2^-8 of the arithmetic's own
 // rounding of that one term).  FP32 entries beyond the factor's reach are
 // exactly zero, which bounds r there; FP64 entries never fall below EPSILON,
-// so r is the whole line once EPSILON X could matter.  A line with a value that
-// is not finite is contracted densely, as an output that is exactly zero in
-// FP64: infinities, NaN and the FP32 factor's zeros then meet as in the
-// dense product.  A result depends on its block's lines only, never on the
+// so r is the whole line once EPSILON X could matter.  An output that is exactly
+// zero in FP64 takes the whole line, and a block with a value that is not
+// finite the whole line in FP64, all of the factor's reach in FP32 and then the
+// zeros beyond it, eight outputs at a time: infinities, NaN and zeros meet
+// as in the dense product.  A result depends on its block's lines only, never on the
 // grid of the launch.
 //
 // Lines are held as 8-byte elements: one FP64 line, or two FP32 lines
@@ -243,19 +244,52 @@ __device__ __forceinline__ void fir8(const typename Vec<T>::V* line, const typen
   }
 }
 
-// The dense sum, for radii past the table (FP32 lines that are not finite).
+// The sum of a block with a value that is not finite, FP32: all of the table's
+// taps, then the zeros beyond them, whose product with that value is NaN, as in
+// the dense sum.  Outputs whose own inputs are all NaN, as every line's are soon
+// after a scaling left the range, are NaN at once (256 x 256, 16 histograms, an
+// evaluation that overflows: dense, with the factor from global memory, 50 ms;
+// without this 17; with it 5.2).  Two inputs at a time in a small loop: written with
+// fir8 (in line, as a call, or as a loop of its own) it cost the finite lines
+// beside it 2 to 4 %.
 template <typename T>
-__device__ __forceinline__ void dense8(const typename Vec<T>::V* line, const Axis<T>& ax, int c0,
-                                       typename Vec<T>::V (&acc)[8]) {
+__device__ __forceinline__ void far8(const typename Vec<T>::V* line, const typename Vec<T>::V* g, const Axis<T>& ax,
+                                     int c0, typename Vec<T>::V (&acc)[8]) {
+  using V = typename Vec<T>::V;
+  bool none = true;  // no output with a number of its own
 #pragma unroll
-  for (int j = 0; j < 8; ++j) acc[j] = typename Vec<T>::V(0);
+  for (int j = 0; j < 8; ++j) {
+    acc[j] = line[c0 + j];
+    T v[Vec<T>::W];
+    Vec<T>::split(acc[j], v);
+    none = none && (c0 + j >= ax.C || (v[0] != v[0] && v[Vec<T>::W - 1] != v[Vec<T>::W - 1]));
+  }
+  if (none) return;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) acc[j] = V(0);
+  V z = V(0);
+  const int lo = c0 + 8 - ax.ext, hi = c0 + ax.ext - 1;  // inputs whose eight entries the table holds
 #pragma unroll 1
-  for (int k = 0; k < ax.C; ++k)
+  for (int k = 0; k < ax.C8; k += 2) {
+    const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(line + k);
+    if (k >= lo && k < hi) {
+      ulonglong2 w[5];  // g[c0 - k - 2 .. c0 - k + 7]
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const int d = abs(c0 + j - k);
-      acc[j] = Vec<T>::fma(line[k], Vec<T>::dup(d < ax.C ? ax.g[d] : T(0)), acc[j]);
+      for (int q = 0; q < 5; ++q) w[q] = *reinterpret_cast<const ulonglong2*>(g + (c0 - k - 2 + 2 * q));
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const int a = j + 2, b = j + 1;  // distances c0 + j - k and c0 + j - k - 1
+        acc[j] = Vec<T>::fma(x.x, (a & 1) ? w[a / 2].y : w[a / 2].x, acc[j]);
+        acc[j] = Vec<T>::fma(x.y, (b & 1) ? w[b / 2].y : w[b / 2].x, acc[j]);
+      }
+    } else {
+      z = Vec<T>::fma(x.x, V(0), z);
+      z = Vec<T>::fma(x.y, V(0), z);
     }
+  }
+  const V one = Vec<T>::dup(T(1));
+#pragma unroll
+  for (int j = 0; j < 8; ++j) acc[j] = Vec<T>::fma(z, one, acc[j]);
 }
 
 // Division of 0 <= i < 65536 by a number that the host knows.
@@ -301,9 +335,14 @@ __device__ __forceinline__ void fir_lines(const typename Vec<T>::V* lines, const
     }
     const int r4 = radius4(ax, (int)__reduce_min_sync(0xffffffffu, (unsigned)(ok ? Vec<T>::bits(m) : 0x7fffffff)), xmag);
     V acc[8];
-    if (r4 <= kPad && r4 + 8 <= ax.ext) fir8<T, false>(lp, g, c0, ax.C8, r4, acc);
-    else if (r4 + 8 <= ax.ext) fir8<T, true>(lp, g, c0, ax.C8, r4, acc);
-    else dense8<T>(lp, ax, c0, acc);
+    if constexpr (sizeof(T) == 8) {  // the table holds a whole line's taps
+      if (r4 <= kPad) fir8<T, false>(lp, g, c0, ax.C8, r4, acc);
+      else fir8<T, true>(lp, g, c0, ax.C8, r4, acc);
+    } else {
+      if (r4 <= kPad && r4 + 8 <= ax.ext) fir8<T, false>(lp, g, c0, ax.C8, r4, acc);
+      else if (r4 + 8 <= ax.ext) fir8<T, true>(lp, g, c0, ax.C8, r4, acc);
+      else far8<T>(lp, g, ax, c0, acc);
+    }
     if (ok) sink(line, c0, acc, ext);
   }
 }
