@@ -928,16 +928,20 @@ bool band_fits(const wdl_ctx* ctx, int K) {
   }
   return true;
 }
-// Taps of a group of eight outputs over data of a few bits' spread against the
-// dense split-BF16 axis passes of grids above 128 (272 x 240, 8 histograms, K = 4,
-// L = 50): 8.6 against 11.2 ms at gamma 25 (72 taps), 11.4 against 12.5 at 80
-// (120), 12.6 against 12.5 at 120 (144), 14.7 against 13.2 at 200 (176); one
-// histogram 3.9 against 5.7 ms at gamma 100.
+// FP32 band sums against the split-BF16 axis passes, on grids above 128 and volumes:
+// by the taps of a group of eight outputs over data of a few bits' spread.  The
+// rule knows the context only (a histogram's bits may not depend on the batch), so
+// the line lies where no batch loses.  At 72 taps (gamma 25), band against axis ms an
+// evaluation: 32 of 200 x 200, K = 4, L = 20 8.4 / 9.1, 48 of 200 x 128, L = 10 3.70 /
+// 3.79, 32 of 272 x 272, L = 20 14.4 / 16.5, 12 of 72^3, L = 6 11.1 / 11.8, one of 272 x 272
+// 1.4 / 2.5; beyond it: 200 x 128 at 80 taps 3.92 / 3.78, 200 x 200 at 88 9.3 / 9.1 and at
+// 136 11.8 / 10.4, 6 of 128^3 at 128 42.5 / 32.9 (one histogram would still win).
+// Lines of up to 48 values are cheap at any width: 32 of 48^3 7.5 / 8.7, 64 of 24^3
+// 1.9 / 3.6; 12 of 72^3 with all taps 14.0 / 11.8.
 bool band_narrow(const wdl_ctx* ctx) {
   for (int a = 0; a < ctx->ndim; ++a) {
     const Axis<float> ax = make_axis<float>(ctx, a);
-    const int r4 = ((int)std::ceil(std::sqrt((double)ax.k1 * (ax.base + 2))) + 3) & ~3;
-    if (std::min(ax.C8, 8 + 2 * std::min(r4, ax.C8)) > 144) return false;
+    if (ax.C8 > 48 && std::sqrt((double)ax.k1 * (ax.base + 2)) > 32.0) return false;
   }
   return true;
 }
