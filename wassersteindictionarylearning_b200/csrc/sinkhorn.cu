@@ -15,6 +15,7 @@
 // in FP64.
 #include <cooperative_groups.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <functional>
@@ -205,13 +206,19 @@ __global__ void k_wloss(const T* __restrict__ v1, const double* __restrict__ v2,
 // The reverse passes' per-(p, k) dot products are summed in two levels with a
 // fixed order: blocks over segments of each image write partial sums,
 // k_add_partials (a warp per (p, k)) adds them.  The segments depend only on N,
-// so a histogram's result does not depend on P or K.  They are 2048 elements, or where that makes fewer than 32 of them a 32nd of the
-// image in whole rounds of 64, so that few small histograms do not leave most SMs
-// without a block (two of 61 x 84, K = 3, FP64, the log domain's fused reverse step: 73 -> 8.3 us).
+// so a histogram's result does not depend on P or K.  They are 2048 elements, or
+// where that makes fewer than 32 of them a 32nd of the image in whole rounds of 64,
+// so that few small histograms do not leave most SMs without a block (two of
+// 61 x 84, K = 3, FP64, the log domain's fused reverse step: 73 -> 8.3 us).  The
+// kernels with a block per (p, k) and segment take no more threads than a segment
+// has elements: 64 histograms of 32 x 32, K = 40, L = 6, log domain, FP32, 2.57 ms
+// an evaluation with 256 threads, 2.39 with 64 (the same bits; 2.33 where
+// one block took the whole image).
 __host__ __device__ inline size_t seg_elems(size_t N) {
   return N >= 65536 ? 2048 : ((N + 31) / 32 + 63) / 64 * 64;
 }
 inline size_t n_segments(size_t N) { return (N + seg_elems(N) - 1) / seg_elems(N); }
+inline unsigned seg_threads(size_t N) { return (unsigned)std::min<size_t>(256, seg_elems(N)); }
 
 __global__ void k_add_partials(double* __restrict__ dot, const double* __restrict__ part, int PK,
                                int nseg) {
@@ -871,7 +878,7 @@ int gradient_both_t(wdl_ctx* ctx, int P, int K, int L, int loss_type, const doub
     if (!log_domain) {
       // the first round's pre here; later rounds' pre ran with the previous post
       if (sstep == L || K > kFuseK) {
-        k_bwd_pre<T><<<dim3((unsigned)(P * K), (unsigned)n_segments(N)), 256, 0, s>>>(
+        k_bwd_pre<T><<<dim3((unsigned)(P * K), (unsigned)n_segments(N)), seg_threads(N), 0, s>>>(
             B.n, B.v, b_s, B.gw, B.r, phi_s, B.lam, tmp, u, B.dpart, K, N, dict);
         WDL_LAUNCH_CHECK(ctx);
       }
@@ -906,7 +913,7 @@ int gradient_both_t(wdl_ctx* ctx, int P, int K, int L, int loss_type, const doub
     } else {
       // the first round's pre here; later rounds' pre ran with the previous post
       if (sstep == L || K > kFuseK) {
-        k_lbwd_pre<T><<<dim3((unsigned)(P * K), (unsigned)n_segments(N)), 256, 0, s>>>(
+        k_lbwd_pre<T><<<dim3((unsigned)(P * K), (unsigned)n_segments(N)), seg_threads(N), 0, s>>>(
             B.n, B.v, b_s, B.gw, B.r, phi_s, B.lam, tmp, u, B.sd, B.sw, B.dpart, K, N);
         WDL_LAUNCH_CHECK(ctx);
       }
