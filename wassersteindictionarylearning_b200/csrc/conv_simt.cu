@@ -536,11 +536,13 @@ struct ConvTimer {
 
 template <typename T>
 int conv_stack_simt(wdl_ctx* ctx, const T* in, T* out, T* tmp, size_t nimg, cudaStream_t s) {
+  // The operator between other kernels of an evaluation: the banded passes, but on
+  // small grids the dense ones (band_pays).
   const int W = ctx->W, H = ctx->H, D = ctx->D;
   const size_t N = ctx->N;
   ConvTimer timer(ctx, s, nimg);
   int rc;
-  if (band_fits<T>(ctx, 0)) {
+  if (band_fits<T>(ctx, 0) && band_pays<T>(ctx)) {
     rc = ctx->ndim == 2 ? band_conv<T, T, T>(ctx, in, out, tmp, nullptr, nimg, s)
                         : band_conv<T, T, T>(ctx, in, out, out, tmp, nimg, s);
     if (rc) return rc;

@@ -928,6 +928,30 @@ bool band_fits(const wdl_ctx* ctx, int K) {
   }
   return true;
 }
+// The banded operator inside an evaluation against the dense axis passes.  On a
+// small grid a banded pass is a block or two per image, whose chain (table, lines,
+// maximum, sums) outlasts a dense tile of 64 x 64.  An evaluation with the Wasserstein
+// loss (101 applications for it), 8 histograms, K = 4, L = 4, banded / dense ms: FP32
+// 32 x 32 1.04 / 0.79 at gamma 2, 1.23 / 0.80 at gamma 50; 24 x 64 1.25 / 0.98 and 1.44 /
+// 1.00; 48 x 48 1.10 / 1.05 and 1.41 / 1.08; 56 x 56 1.06 / 1.29 and 1.52 / 1.33; volumes of 24^3
+// 1.81 / 1.25, of 32^3 1.83 / 1.41 and 2.13 / 1.45.  FP64, whose dense passes cost more: 16 x 16
+// 0.90 / 0.70, 32 x 32 1.27 / 1.05, 40 x 40 1.41 / 1.42, 24^3 1.89 / 1.77 against 2.15 for the
+// whole evaluation before the banded kernels.
+template <typename T>
+bool band_pays(const wdl_ctx* ctx) {
+  if (ctx->ndim == 2)
+    return ctx->N > (sizeof(T) == 4 ? 48 * 48 : 32 * 32) || std::max(ctx->W, ctx->H) > 64;
+  bool all_taps = sizeof(T) == 4;  // FP32 volumes: where the sums take a line's every tap
+  for (int a = 0; a < 3; ++a) {
+    const Axis<T> ax = make_axis<T>(ctx, a);
+    const int r4 = ((int)std::ceil(std::min(std::sqrt((double)ax.k1 * (ax.base + 2)), 64.0)) + 3) & ~3;
+    all_taps &= ax.C8 <= 48 && 8 + 2 * r4 >= ax.C8;
+  }
+  return !all_taps;
+}
+template bool band_pays<float>(const wdl_ctx*);
+template bool band_pays<double>(const wdl_ctx*);
+
 // FP32 band sums against the split-BF16 axis passes, on grids above 128 and volumes:
 // by the taps of a group of eight outputs over data of a few bits' spread.  The
 // rule knows the context only (a histogram's bits may not depend on the batch), so

@@ -230,6 +230,9 @@ struct BandEval {
 // Whether the lines of a call fit shared memory (K = 0: the operator alone).
 template <typename T>
 bool band_fits(const wdl_ctx* ctx, int K);
+// Whether the banded operator beats the dense passes between other kernels.
+template <typename T>
+bool band_pays(const wdl_ctx* ctx);
 // Whether the factor is narrow enough for FP32 band sums to beat tensor-core axis passes.
 bool band_narrow(const wdl_ctx* ctx);
 template <typename T>
