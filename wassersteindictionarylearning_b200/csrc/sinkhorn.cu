@@ -1077,13 +1077,15 @@ size_t band_bytes(const wdl_ctx* ctx, size_t P, size_t K, size_t L, bool b_init,
   return plan.off + 256;
 }
 
-// Kernel-domain contexts whose lines fit: those without tensor cores, and those
-// above the fused kernel's grids (sides over 128, volumes) whose factor is narrow
-// enough for the banded FP32 sums to beat the tensor-core axis passes.
+// Kernel-domain contexts whose lines fit and whose sizes suit the fused rows: those
+// without tensor cores, and those above the fused kernel's grids (sides over 128,
+// volumes) whose factor is narrow enough for the banded FP32 sums to beat the
+// tensor-core axis passes.
 bool use_band(const wdl_ctx* ctx, int K) {
   if (ctx->domain != WDL_DOMAIN_KERNEL || tc_fused(ctx)) return false;
   if (ctx->tc && !band_narrow(ctx)) return false;
-  return ctx->precision == WDL_FP64 ? band_fits<double>(ctx, K) : band_fits<float>(ctx, K);
+  return ctx->precision == WDL_FP64 ? band_fits<double>(ctx, K) && band_rows_pay<double>(ctx, K)
+                                    : band_fits<float>(ctx, K) && band_rows_pay<float>(ctx, K);
 }
 
 template <typename T>

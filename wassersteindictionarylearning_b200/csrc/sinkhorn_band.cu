@@ -46,7 +46,8 @@ using namespace band;
 
 constexpr int kMaxThreads = 256, kMaxWarps = kMaxThreads / 32;
 constexpr size_t kSmemMost = 200 * 1024;
-constexpr int kMaxK = 64;  // atoms of one rows block
+// Atoms of one rows block (more: band_rows_pay's first figures).
+constexpr int kMaxK = 32;
 
 template <typename T>
 const T* factor_row(const wdl_ctx* ctx, int axis);
@@ -79,6 +80,20 @@ Axis<T> make_axis(const wdl_ctx* ctx, int axis) {
     if (sizeof(T) == 4 && 4 * (i + 1) >= ax.reach) ax.lim[i] = 1000000;
   }
   return ax;
+}
+
+// The radius that data of a few bits' spread take, and whether it covers every line.
+template <typename T>
+int few_bits_radius4(const Axis<T>& ax) {
+  return ((int)std::ceil(std::min(std::sqrt((double)ax.k1 * (ax.base + 2)), 16384.0)) + 3) & ~3;
+}
+template <typename T>
+bool covers_lines(const wdl_ctx* ctx) {
+  for (int a = 0; a < ctx->ndim; ++a) {
+    const Axis<T> ax = make_axis<T>(ctx, a);
+    if (8 + 2 * few_bits_radius4(ax) < ax.C8) return false;
+  }
+  return true;
 }
 
 // Lines of a block: about 160 eight-output items per pass (a power of two of
@@ -928,6 +943,31 @@ bool band_fits(const wdl_ctx* ctx, int K) {
   }
   return true;
 }
+// The fused rows and columns kernels of an evaluation against separate kernels around
+// the operator, on sizes and the factor alone (a histogram's bits may not depend on
+// the batch).  A rows block's chain of K logarithms and divisions a pixel, and its line
+// buffers for K atoms, lose where there are many atoms or hardly a pixel; on
+// short lines that the factor covers whole, the sums have no tap to leave out either.
+// Banded rows / separate kernels / before the banded kernels, ms an evaluation, L = 6 or 8:
+//   atoms x groups of eight: 8 of 64 x 64, K = 64, FP64 4.1 / 2.6 / 3.0; 8 of 32^3, K = 64
+//     33.6 / 19.4 / 23.9; gamma 50, FP64: 64 of 64 x 64 K = 12 2.71 / 2.80 / 2.81, K = 16 3.85 /
+//     3.57 / 3.58; 8 of 40^3 K = 8 4.40 / 4.98 / 5.10, K = 20 15.5 / 12.4 / 11.8
+//   pixels: one histogram, K = 5, FP32 16 x 16 0.39 / 0.25 / 0.27, 32 x 32 0.30 / 0.31 / 0.41
+//   shared memory, one block on an SM: 24 of 128 x 128, K = 24, FP64 8.6 / 5.3 / 11.7, at gamma
+//     50 12.0 / 7.9 / 11.7; few atoms on long lines want it: 2048 x 64, K = 2 0.46 / 0.68 / 6.3
+template <typename T>
+bool band_rows_pay(const wdl_ctx* ctx, int K) {
+  const RowsShape<T> sh(ctx, K);
+  const bool vol = ctx->ndim == 3;
+  if (std::max({ctx->W, ctx->H, ctx->D}) > 64) return K <= 16 || sh.bwd_smem(K) <= 110 * 1024;
+  if (ctx->N < (sizeof(T) == 4 ? 1024 : vol ? 513 : 257)) return false;
+  const int items = K * sh.ax.G;
+  if (!covers_lines<T>(ctx)) return items <= (vol ? 80 : 192);
+  return items <= (!vol ? 96 : sh.ax.G <= 4 ? 80 : 48);
+}
+template bool band_rows_pay<float>(const wdl_ctx*, int);
+template bool band_rows_pay<double>(const wdl_ctx*, int);
+
 // The banded operator inside an evaluation against the dense axis passes.  On a
 // small grid a banded pass is a block or two per image, whose chain (table, lines,
 // maximum, sums) outlasts a dense tile of 64 x 64.  An evaluation with the Wasserstein
@@ -935,19 +975,14 @@ bool band_fits(const wdl_ctx* ctx, int K) {
 // 32 x 32 1.04 / 0.79 at gamma 2, 1.23 / 0.80 at gamma 50; 24 x 64 1.25 / 0.98 and 1.44 /
 // 1.00; 48 x 48 1.10 / 1.05 and 1.41 / 1.08; 56 x 56 1.06 / 1.29 and 1.52 / 1.33; volumes of 24^3
 // 1.81 / 1.25, of 32^3 1.83 / 1.41 and 2.13 / 1.45.  FP64, whose dense passes cost more: 16 x 16
-// 0.90 / 0.70, 32 x 32 1.27 / 1.05, 40 x 40 1.41 / 1.42, 24^3 1.89 / 1.77 against 2.15 for the
-// whole evaluation before the banded kernels.
+// 0.90 / 0.70, 32 x 32 1.27 / 1.05, 40 x 40 1.41 / 1.42; volumes of 16^3 1.31 / 1.20,
+// of 24^3 with 64 histograms 4.7 / 5.4.
 template <typename T>
 bool band_pays(const wdl_ctx* ctx) {
   if (ctx->ndim == 2)
     return ctx->N > (sizeof(T) == 4 ? 48 * 48 : 32 * 32) || std::max(ctx->W, ctx->H) > 64;
-  bool all_taps = sizeof(T) == 4;  // FP32 volumes: where the sums take a line's every tap
-  for (int a = 0; a < 3; ++a) {
-    const Axis<T> ax = make_axis<T>(ctx, a);
-    const int r4 = ((int)std::ceil(std::min(std::sqrt((double)ax.k1 * (ax.base + 2)), 64.0)) + 3) & ~3;
-    all_taps &= ax.C8 <= 48 && 8 + 2 * r4 >= ax.C8;
-  }
-  return !all_taps;
+  // volumes: where the sums take a line's every tap
+  return std::max({ctx->W, ctx->H, ctx->D}) > (sizeof(T) == 4 ? 48 : 16) || !covers_lines<T>(ctx);
 }
 template bool band_pays<float>(const wdl_ctx*);
 template bool band_pays<double>(const wdl_ctx*);

@@ -230,6 +230,9 @@ struct BandEval {
 // Whether the lines of a call fit shared memory (K = 0: the operator alone).
 template <typename T>
 bool band_fits(const wdl_ctx* ctx, int K);
+// Whether the fused banded kernels of an evaluation beat separate kernels around the operator.
+template <typename T>
+bool band_rows_pay(const wdl_ctx* ctx, int K);
 // Whether the banded operator beats the dense passes between other kernels.
 template <typename T>
 bool band_pays(const wdl_ctx* ctx);
