@@ -282,12 +282,15 @@ int wdl_convolve_device_noalloc(wdl_ctx* ctx, const double* u, double* out, int 
 
 /* ---- Instrumentation ------------------------------------------------------------
  * Kernel launches issued by this context since creation (every kernel of this
- * library counts one), and the time in the dominant kernel (the separable
- * operator, or the fused Sinkhorn kernel on the tensor-core path) measured with
- * CUDA events on the launching stream since profiling was switched on
- * (level >= 1; the events synchronise each launch); conv_images counts the
+ * library counts one), and the time in the dominant kernels measured with CUDA
+ * events on the launching stream since profiling was switched on (level >= 1;
+ * the events synchronise each launch): the separable operator where it runs on its
+ * own (one launch an application on a stack of images), the fused Sinkhorn kernel
+ * on the tensor-core path, or the banded CUDA-core kernels of an evaluation's
+ * forward and reverse passes (one launch each), the last two with the
+ * elementwise steps that are fused with the operator; conv_images counts the
  * separable-operator applications those launches performed (an image through
- * both axes is one).  Level 2 also records a
+ * every axis is one).  Level 2 also records a
  * device-side phase trace of the fused kernel: wdl_phase_trace returns 27
  * values, for item types forward / dictionary / weights, 8 accumulated phase
  * times in ns (claim, dependency wait, prologue, first operator, mid step,

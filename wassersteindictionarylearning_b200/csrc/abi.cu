@@ -123,7 +123,12 @@ int convolve_dev_t(wdl_ctx* ctx, const double* u, double* out, int nv, cudaStrea
   T* b = ctx->arena.take<T>(n);
   T* t = ctx->arena.take<T>(n);
   // CUDA-core contexts convert on the way in and out of the passes themselves
-  if (!ctx->tc && band_fits<T>(ctx, 0)) return band_conv<double, T, double>(ctx, u, out, a, b, nv, s);
+  if (!ctx->tc && band_fits<T>(ctx, 0)) {
+    PassTimer timer(ctx, s);
+    if ((rc = band_conv<double, T, double>(ctx, u, out, a, b, nv, s))) return rc;
+    timer.done(nv);
+    return WDL_OK;
+  }
   const unsigned G = grid_for(n, 256, ctx->sm_count);
   k_to_t<T><<<G, 256, 0, s>>>(u, a, n);
   WDL_LAUNCH_CHECK(ctx);

@@ -891,27 +891,6 @@ int plane_cols(wdl_ctx* ctx, const T* in, TO* out, size_t nimg, int im0, cudaStr
 
 }  // namespace
 
-// wdl_conv_profile of a pass over the iterations: the operator is fused with the steps
-// between its applications, so the whole pass counts as one launch of `apps`
-// applications, as the fused tensor-core kernel's does.
-struct PassTimer {
-  wdl_ctx* ctx;
-  cudaStream_t s;
-  PassTimer(wdl_ctx* c, cudaStream_t st) : ctx(c), s(st) {
-    if (ctx->profiling) cudaEventRecord(ctx->ev_a, s);
-  }
-  void done(double apps) {
-    if (!ctx->profiling) return;
-    cudaEventRecord(ctx->ev_b, s);
-    cudaEventSynchronize(ctx->ev_b);
-    float ms = 0;
-    cudaEventElapsedTime(&ms, ctx->ev_a, ctx->ev_b);
-    ctx->conv_ms += ms;
-    ctx->conv_launches += 1;
-    ctx->conv_images += apps;
-  }
-};
-
 // The shape of a rows launch.
 template <typename T>
 struct RowsShape {

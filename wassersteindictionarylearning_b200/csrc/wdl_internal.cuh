@@ -210,6 +210,27 @@ inline int log_conv_stack<double>(wdl_ctx* ctx, const double* in, double* out, d
   return log_conv_stack_f64(ctx, in, out, tmp, nimg, is, os, ts, s, sf, so, sp);
 }
 
+// wdl_conv_profile of the banded kernels.  In an evaluation the operator is fused with
+// the steps between its applications, so a whole pass over the iterations counts as
+// one launch of `apps` applications, as the fused tensor-core kernel's does.
+struct PassTimer {
+  wdl_ctx* ctx;
+  cudaStream_t s;
+  PassTimer(wdl_ctx* c, cudaStream_t st) : ctx(c), s(st) {
+    if (ctx->profiling) cudaEventRecord(ctx->ev_a, s);
+  }
+  void done(double apps) {
+    if (!ctx->profiling) return;
+    cudaEventRecord(ctx->ev_b, s);
+    cudaEventSynchronize(ctx->ev_b);
+    float ms = 0;
+    cudaEventElapsedTime(&ms, ctx->ev_a, ctx->ev_b);
+    ctx->conv_ms += ms;
+    ctx->conv_launches += 1;
+    ctx->conv_images += apps;
+  }
+};
+
 // ---- banded CUDA-core forms (sinkhorn_band.cu) ---------------------------------------
 // One kernel-domain evaluation's device buffers: atoms [K][N], lam [P][K] in T
 // and FP64, the iterate store (conv_b, phi [L][P][K][N] and bary [L][P][N]; a
