@@ -63,7 +63,7 @@ struct LogFitProblem {
   float *u, *r;          // [K][N]
   float *gw, *blog;      // [N]
   uint8_t *sw, *ts;      // [K][N] signs and intermediate signs
-  double* part;          // [group][K + 1] partial sums (dot products, loss)
+  double* part;          // [kMostGroup][K + 1] partial sums (dot products, loss)
   double* v;             // L-BFGS vectors (pool_doubles(K))
   double* w64;           // [K] weights of the current trial point
   float* w32;
@@ -201,6 +201,11 @@ __global__ void __launch_bounds__(kLfThreads)
   const int K = p.K, L = p.L, tid = threadIdx.x;
   const size_t N = (size_t)p.W * p.H, KN = (size_t)K * N;
   const size_t gstride = (size_t)G * kLfThreads, g0 = (size_t)rank * kLfThreads + tid;
+  // The FP64 sums (loss, dot products) are those of kMostGroup CTAs whatever the group:
+  // a CTA stands for kVirtual of them in turn, so a fit's bits do not depend on the
+  // other problems of the call, which size the group.
+  constexpr int kVirtual = kMostGroup / G;
+  constexpr size_t vstride = (size_t)kMostGroup * kLfThreads;
 
   for (int e = 0; e < max_evals; ++e) {
     group_sync<G>();
@@ -228,48 +233,56 @@ __global__ void __launch_bounds__(kLfThreads)
       group_sync<G>();
     }
     // ---- loss and its gradient (cpp/loss.h:19-90); gw = g * bary (:633-635) --------
-    double lacc = 0;
-    for (size_t j = g0; j < N; j += gstride) {
-      const float v1 = expf(p.blog[j]);
-      const double o = p.obs[j];
-      const float v2 = (float)o;
-      float g;
-      if (p.loss_type == WDL_LOSS_TV) {
-        lacc += fabs((double)v1 - o);
-        g = v1 - v2 > 0.f ? 0.5f : -0.5f;
-      } else if (p.loss_type == WDL_LOSS_QUADRATIC) {
-        const double d = (double)v1 - o;
-        lacc += d * d;
-        g = 2.f * (v1 - v2);
-      } else {
-        const double rr = (double)v1 / o;
-        lacc += (double)v1 * log(rr > kEpsilon ? rr : kEpsilon) - (double)v1 + o;
-        const float q2 = v1 / v2;
-        g = q2 > 0.f ? logf(q2) : (float)kLogEpsilon;
+    for (int m = 0; m < kVirtual; ++m) {
+      const size_t j0 = g0 + m * gstride;
+      if (j0 - tid >= N) break;  // uniform over the CTA
+      double lacc = 0;
+      for (size_t j = j0; j < N; j += vstride) {
+        const float v1 = expf(p.blog[j]);
+        const double o = p.obs[j];
+        const float v2 = (float)o;
+        float g;
+        if (p.loss_type == WDL_LOSS_TV) {
+          lacc += fabs((double)v1 - o);
+          g = v1 - v2 > 0.f ? 0.5f : -0.5f;
+        } else if (p.loss_type == WDL_LOSS_QUADRATIC) {
+          const double d = (double)v1 - o;
+          lacc += d * d;
+          g = 2.f * (v1 - v2);
+        } else {
+          const double rr = (double)v1 / o;
+          lacc += (double)v1 * log(rr > kEpsilon ? rr : kEpsilon) - (double)v1 + o;
+          const float q2 = v1 / v2;
+          g = q2 > 0.f ? logf(q2) : (float)kLogEpsilon;
+        }
+        p.gw[j] = g * v1;
       }
-      p.gw[j] = g * v1;
+      lacc = block_sum_d(lacc, sh);
+      if (tid == 0) p.part[(m * G + rank) * (K + 1) + K] = lacc;
     }
-    lacc = block_sum_d(lacc, sh);
-    if (tid == 0) p.part[rank * (K + 1) + K] = lacc;
     // ---- reverse pass, weight recursion (:730-812) -------------------------------------
     for (size_t i = g0; i < KN; i += gstride) p.r[i] = 0.f;
-    double dacc[kLfMaxK];
-    for (int k = 0; k < K; ++k) dacc[k] = 0;
+    double dacc[kLfMaxK * kVirtual];
+    for (int i = 0; i < K * kVirtual; ++i) dacc[i] = 0;
     group_sync<G>();
     for (int s = L; s >= 1; --s) {
       const float* phs = p.tphi + (size_t)(s - 1) * KN;
       for (int k = 0; k < K; ++k) {
         const float l = s_lam[k];
-        double acc = 0;
-        for (size_t j = g0; j < N; j += gstride) {
-          const size_t i = k * N + j;
-          const float ph = phs[i], g = p.gw[j];
-          acc += (double)ph * (double)g;
-          const float y = l * g + p.r[i];
-          p.sw[i] = y >= 0.f;
-          p.u[i] = logf(fabsf(y)) - ph;
+        for (int m = 0; m < kVirtual; ++m) {
+          const size_t j0 = g0 + m * gstride;
+          if (j0 >= N) break;
+          double acc = 0;
+          for (size_t j = j0; j < N; j += vstride) {
+            const size_t i = k * N + j;
+            const float ph = phs[i], g = p.gw[j];
+            acc += (double)ph * (double)g;
+            const float y = l * g + p.r[i];
+            p.sw[i] = y >= 0.f;
+            p.u[i] = logf(fabsf(y)) - ph;
+          }
+          dacc[k * kVirtual + m] += acc;
         }
-        dacc[k] += acc;
       }
       group_sync<G>();
       if (s == 1) break;
@@ -290,16 +303,20 @@ __global__ void __launch_bounds__(kLfThreads)
       }
       group_sync<G>();
     }
-    for (int k = 0; k < K; ++k) {
-      const double t = block_sum_d(dacc[k], sh);
-      if (tid == 0) p.part[rank * (K + 1) + k] = t;
+    for (int m = 0; m < kVirtual; ++m) {
+      if (g0 + m * gstride - tid >= N) break;
+      for (int k = 0; k < K; ++k) {
+        const double t = block_sum_d(dacc[k * kVirtual + m], sh);
+        if (tid == 0) p.part[(m * G + rank) * (K + 1) + k] = t;
+      }
     }
     group_sync<G>();
     // ---- one L-BFGS step (rank 0, thread 0) -----------------------------------------
     if (rank == 0 && tid == 0) {
+      const int parts = (int)min((size_t)kMostGroup, (N + kLfThreads - 1) / kLfThreads);
       for (int k = 0; k <= K; ++k) {
         double t = 0;
-        for (int g = 0; g < G; ++g) t += p.part[g * (K + 1) + k];
+        for (int g = 0; g < parts; ++g) t += p.part[g * (K + 1) + k];
         s_la[k] = t;
       }
       const double f = p.loss_type == WDL_LOSS_TV ? 0.5 * s_la[K] : s_la[K];
