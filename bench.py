@@ -341,9 +341,10 @@ def run_ours(args):
             if key6[0] == 2:  # tensor-core axis pass: output tile height
                 tuned.append(dict(kind="tc_axis_pass", rows=key6[1], row_len=key6[2], images=key6[3],
                                   tile_rows=choice.value, ms=round(tms.value, 4)))
-            else:  # log-domain axis pass: rows per block
+            else:  # log-domain axis pass: rows per block, outputs per thread
                 tuned.append(dict(kind="log_axis_pass", rows=key6[1], row_len=key6[2], images=key6[3],
                                   signed=bool(key6[5]), rows_per_block=choice.value,
+                                  outputs_per_thread=L_.wdl_autotune_outputs(ctx, i),
                                   ms=round(tms.value, 4)))
     peaks = {}
     try:

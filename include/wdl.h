@@ -305,14 +305,17 @@ int wdl_conv_profile(const wdl_ctx* ctx, double* conv_ms, long long* conv_launch
  * rows, row length, images, element bytes, signed} (kind 1 = log-domain axis
  * pass: variant = rows per block; kind 2 = tensor-core axis pass: variant =
  * output tile height, element bytes 2 for split BF16 and 4 for TF32), the
- * chosen variant and its time in ms.  wdl_autotune_count returns the number of
- * entries.  wdl_set_autotune(ctx, 0) stops this context from timing variants
+ * chosen variant and its time in ms.  wdl_autotune_outputs returns the outputs
+ * of a row that a thread of the chosen log-domain variant makes: 4, or 1 for the form for
+ * small launches (8 rows per block, as a variant of 4 may have too); 0 for other
+ * kinds.  wdl_autotune_count returns the number of entries.  wdl_set_autotune(ctx, 0) stops this context from timing variants
  * on first calls (a latency-bound caller such as a request loop, where every
  * timing would also synchronise the stream); untuned shapes then take the
  * default variant.  On by default; WDL_AUTOTUNE=0 turns it off process-wide. */
 int wdl_set_autotune(wdl_ctx* ctx, int on);
 int wdl_autotune_count(const wdl_ctx* ctx);
 int wdl_autotune_entry(const wdl_ctx* ctx, int i, long long* key6, int* choice, float* ms);
+int wdl_autotune_outputs(const wdl_ctx* ctx, int i);
 /* Failure detection of the fused tensor-core kernel (no reference counterpart;
  * the reference's only failure signal is a NaN loss that cancels L-BFGS,
  * cpp/inverseWasserstein.h:1180-1184).  Every wait of that kernel on another

@@ -108,6 +108,7 @@ SIGNATURES = {
                                 C.c_int),
     "wdl_inject_fault": ([_vp, C.c_int], C.c_int),
     "wdl_autotune_count": ([_vp], C.c_int),
+    "wdl_autotune_outputs": ([_vp, C.c_int], C.c_int),
     "wdl_autotune_entry": ([_vp, C.c_int, C.POINTER(C.c_longlong), C.POINTER(C.c_int),
                             C.POINTER(C.c_float)], C.c_int),
 }

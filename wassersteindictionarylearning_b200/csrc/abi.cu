@@ -348,6 +348,12 @@ int wdl_autotune_entry(const wdl_ctx* ctx, int i, long long* key6, int* choice, 
   return WDL_OK;
 }
 
+int wdl_autotune_outputs(const wdl_ctx* ctx, int i) {
+  if (!ctx || i < 0 || i >= (int)ctx->tuned.size()) return WDL_ERR_INVALID_ARG;
+  const auto& e = ctx->tuned[i];
+  return e.key[0] != 1 ? 0 : e.lanes ? 1 : 4;
+}
+
 int wdl_exp_profile(const wdl_ctx* ctx, double* executed_exps) {
   if (!ctx || !executed_exps) return WDL_ERR_INVALID_ARG;
   *executed_exps = ctx->log_exps;
