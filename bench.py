@@ -27,6 +27,7 @@ from __future__ import annotations
 import argparse
 import ctypes as C
 import json
+import math
 import os
 import statistics
 import subprocess
@@ -353,6 +354,15 @@ def run_ours(args):
         pass
     flop_per_img = 2.0 * N * (W + H)  # dense separable contraction, both axes
     products = 3 if precision == "split_bf16" else 1
+    # CUDA-core evaluations, and tensor-core contexts above the fused kernel's grids whose
+    # factor is narrow (no axis pass was tuned), sum only the taps that reach the
+    # arithmetic's rounding: those are counted, the dense contraction beside them
+    banded = wl["domain"] != "log" and (precision in ("fp32", "fp64") or (
+        max(W, H) > 128 and not any(t["kind"] == "tc_axis_pass" for t in tuned)))
+    dense_per_img = flop_per_img
+    if banded:
+        reach = math.ceil(math.sqrt(wl["gamma"] * (53 if precision == "fp64" else 24) * math.log(2.0)))
+        flop_per_img, products = 2.0 * N * sum(min(m, 2 * reach + 1) for m in (W, H)), 1
     conv_launch_ms = conv_ms.value / max(conv_launches.value, 1)
     imgs_per_launch = conv_imgs.value / max(conv_launches.value, 1)
     # algorithmic (useful) FLOPs: one dense contraction per operator application;
@@ -383,7 +393,7 @@ def run_ours(args):
                         reference_equivalent_texp_s=ref_rate,
                         executed_exp_share=exps.value / max(conv_imgs.value * N * (W + H), 1),
                         conv_share_of_step=conv_ms.value / (ms / args.steps))
-    elif precision in ("split_bf16", "tf32"):
+    elif precision in ("split_bf16", "tf32") and not banded:
         peak = peaks.get("bf16_tflops", 1590.0) * (0.5 if precision == "tf32" else 1.0)
         peak_src = "of measured bf16 burst" if peaks else "of fallback"
         bound = "tensor"
@@ -392,7 +402,7 @@ def run_ours(args):
         mhz = peaks.get("sm_max_mhz", 1965.0)
         peak = 148 * 128 * 2 * mhz * 1e6 / 1e12 / (2.0 if precision == "fp64" else 1.0)
         peak_src = "of nominal CUDA-core FMA peak at max clock"
-        bound = "fp32-cuda-core" if precision == "fp32" else "fp64-cuda-core"
+        bound = "fp64-cuda-core" if precision == "fp64" else "fp32-cuda-core"
     if wl["domain"] != "log":
         # DRAM bytes (read + write) of one fused launch at P=64, L=100, from a
         # one-pass ncu capture of this workload, scaled by P*L
@@ -400,12 +410,16 @@ def run_ours(args):
                    if wl["name"] == "batched128" and precision == "split_bf16" else None)
         roofline = dict(bound=bound, achieved=achieved_tflops, peak=peak, unit="TFLOP/s",
                         frac=achieved_tflops / peak, traffic=traffic, peak_source=peak_src,
-                        algorithmic_bytes_per_launch=8.0 * K * N * 4 * P * L,
+                        # banded: a launch is the forward or the reverse half
+                        algorithmic_bytes_per_launch=8.0 * K * N * 4 * P * L / (2 if banded else 1),
                         executed_tflops=achieved_tflops * products,
+                        dense_equivalent_tflops=achieved_tflops * dense_per_img / flop_per_img,
                         ceiling_frac=1.0 / products,
                         kernel=(f"fused Sinkhorn kernel: one launch = {imgs_per_launch:.0f} separable-operator "
                                 "applications (whole forward + reverse pass)"
                                 if precision in ("split_bf16", "tf32") and W <= 128 and H <= 128
+                                else f"banded CUDA-core kernels, a forward or reverse pass: {imgs_per_launch:.0f} "
+                                     "operator applications with the steps between them" if banded
                                 else f"separable Gaussian operator ({'tensor-core axis passes' if precision in ('split_bf16', 'tf32') else 'CUDA cores'}): "
                                      f"one launch = {imgs_per_launch:.0f} images"),
                         conv_share_of_step=conv_ms.value / (ms / args.steps))
