@@ -22,7 +22,7 @@
 //
 // Lines are held as 8-byte elements: one FP64 line, or two FP32 lines
 // interleaved, whose sums advance together on the packed FP32 multiply-add
-// (half the issue slots; the kernels are bound by issue).
+// (half the issue slots of the sums).
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>

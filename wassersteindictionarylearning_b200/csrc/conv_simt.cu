@@ -6,7 +6,9 @@
 // three such passes (:762-807).  Here every pass is the same primitive: an
 // image viewed as [R][C] (C contiguous) is contracted along C with the dense
 // C x C factor and written as [C][R], moving the contracted axis to the front.
-// Applying it once per axis returns the image to its original layout.
+// Applying it once per axis returns the image to its original layout.  Most calls
+// take the banded passes of sinkhorn_band.cu instead: the dense ones serve small
+// grids and lines too long for a block's shared memory.
 #include <algorithm>
 #include <cstdlib>
 #include <cstring>

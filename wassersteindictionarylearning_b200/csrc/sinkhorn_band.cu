@@ -23,11 +23,13 @@
 // gamma 1, FP32 69.4 -> 20.3 ms an evaluation; 16 of 64 x 64, K = 4, L = 25, FP32
 // 2.38 -> 0.84 ms (350 -> 100 launches); one of 161 x 161, K = 5, L = 50, FP64,
 // weights only 10.9 -> 2.2 ms.  The dense passes spent 128 taps where 13 reach
-// the FP32 rounding; here the kernels are bound by issue (a quarter of the
-// instructions at 128 x 128 are the sums' packed multiply-adds, the rest the
-// logarithms, divisions, staging and addresses) and, for few histograms, by each
-// launch's latency.  Tiles that lie inside the image and are whole groups of eight
-// take a form without edge tests (24.4 -> 21.4 ms at 128 x 128).
+// the FP32 rounding; here a quarter of the instructions at 128 x 128 are the sums'
+// packed multiply-adds, the rest the logarithms, divisions, staging and addresses,
+// and with 80 registers and 21 warps an SM their issue slots are 51 to 59 % busy: the latency
+// of dependent instructions and of the loads before each sum bounds them, and for
+// few histograms each launch's chain in one block an SM (9 to 17 % busy).  Tiles that
+// lie inside the image and are whole groups of eight take a form without edge tests
+// (24.4 -> 21.4 ms at 128 x 128).
 //
 // The blocks' shapes depend on the grid, K and the type only, so a
 // histogram's results are the same bits in any batch.

@@ -357,9 +357,9 @@ struct BatchPlan {
 // device); reserves extra_bytes at plan.extra_off for the caller.
 int batch_prepare(wdl_ctx* ctx, const wdl_problem* pb, int nprob, size_t extra_bytes, BatchPlan& bp,
                   cudaStream_t s);
-// Work items by round (every problem's forward iteration r, then its reverse
-// step 2L-r), for the histograms whose flag in `active` is set (flattened
-// problem by problem; null = all).
+// Work items, a problem's forward iterations and then its reverse steps in order,
+// the problems merged in proportion to their rounds, for the histograms whose flag in
+// `active` is set (flattened problem by problem; null = all).
 void batch_items(const BatchPlan& bp, const std::vector<uint8_t>* active, std::vector<int4>& items);
 // Clears the accumulated buffers and launches the fused kernel over the first
 // n_items entries of the item table at plan.items_off.
