@@ -115,6 +115,8 @@ struct wdl_ctx {
   };
   std::vector<GraphEntry> graphs;
 
+  // Host staging of the many-problem calls (batch.cu): their small inputs, their outputs.
+  std::vector<char> batch_in, batch_out;
   // Autotuned launch shapes (conv_simt.cu): key -> chosen variant.
   struct TuneEntry {
     long long key[6];
