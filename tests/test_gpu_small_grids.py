@@ -15,7 +15,7 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("precision", ["fp32", "fp64"])
 @pytest.mark.parametrize("W,H,D,gamma", [
     (1, 9, 1, 2.0), (32, 32, 1, 2.0), (33, 32, 1, 2.0), (48, 48, 1, 40.0), (49, 48, 1, 40.0), (24, 64, 1, 9.0),
-    (65, 24, 1, 9.0), (12, 10, 9, 4.0), (20, 17, 40, 2.0), (48, 7, 8, 60.0)])
+    (65, 24, 1, 9.0), (64, 50, 1, 40.0), (12, 10, 9, 4.0), (20, 17, 40, 2.0), (48, 7, 8, 60.0)])
 def test_wasserstein_loss_around_the_line(oracle, W, H, D, gamma, precision):
     from wassersteindictionarylearning_b200 import (CudaGaussian2DKernel, CudaGaussian3DKernel, Problem,
                                                     WassersteinRegression)

@@ -933,7 +933,8 @@ bool band_fits(const wdl_ctx* ctx, int K) {
 //   atoms x groups of eight: 8 of 64 x 64, K = 64, FP64 4.1 / 2.6 / 3.0; 8 of 32^3, K = 64
 //     33.6 / 19.4 / 23.9; gamma 50, FP64: 64 of 64 x 64 K = 12 2.71 / 2.80 / 2.81, K = 16 3.85 /
 //     3.57 / 3.58; 8 of 40^3 K = 8 4.40 / 4.98 / 5.10, K = 20 15.5 / 12.4 / 11.8
-//   pixels: one histogram, K = 5, FP32 16 x 16 0.39 / 0.25 / 0.27, 32 x 32 0.30 / 0.31 / 0.41
+//   pixels: one histogram, K = 5, FP32 16 x 16 0.39 / 0.25 / 0.27, 32 x 32 0.30 / 0.31 / 0.41;
+//     barycenters of 16^3, K = 8, L = 20 0.56 / 0.48 / 0.48
 //   shared memory, one block on an SM: 24 of 128 x 128, K = 24, FP64 8.6 / 5.3 / 11.7, at gamma
 //     50 12.0 / 7.9 / 11.7; few atoms on long lines want it: 2048 x 64, K = 2 0.46 / 0.68 / 6.3
 template <typename T>
@@ -941,7 +942,7 @@ bool band_rows_pay(const wdl_ctx* ctx, int K) {
   const RowsShape<T> sh(ctx, K);
   const bool vol = ctx->ndim == 3;
   if (std::max({ctx->W, ctx->H, ctx->D}) > 64) return K <= 16 || sh.bwd_smem(K) <= 110 * 1024;
-  if (ctx->N < (sizeof(T) == 4 ? 1024 : vol ? 513 : 257)) return false;
+  if (ctx->N < (sizeof(T) == 4 ? (vol ? 4097 : 1024) : vol ? 513 : 257)) return false;
   const int items = K * sh.ax.G;
   if (!covers_lines<T>(ctx)) return items <= (vol ? 80 : 192);
   return items <= (!vol ? 96 : sh.ax.G <= 4 ? 80 : 48);
@@ -954,14 +955,18 @@ template bool band_rows_pay<double>(const wdl_ctx*, int);
 // maximum, sums) outlasts a dense tile of 64 x 64.  An evaluation with the Wasserstein
 // loss (101 applications for it), 8 histograms, K = 4, L = 4, banded / dense ms: FP32
 // 32 x 32 1.04 / 0.79 at gamma 2, 1.23 / 0.80 at gamma 50; 24 x 64 1.25 / 0.98 and 1.44 /
-// 1.00; 48 x 48 1.10 / 1.05 and 1.41 / 1.08; 56 x 56 1.06 / 1.29 and 1.52 / 1.33; volumes of 24^3
-// 1.81 / 1.25, of 32^3 1.83 / 1.41 and 2.13 / 1.45.  FP64, whose dense passes cost more: 16 x 16
+// 1.00; 48 x 48 1.10 / 1.05 and 1.41 / 1.08; 56 x 56 1.06 / 1.29 and 1.52 / 1.33, where at
+// gamma 50 the sums take a line's every tap; volumes of 24^3 1.81 / 1.25, of 32^3 1.83 / 1.41 and
+// 2.13 / 1.45.  FP64, whose dense passes cost more: 16 x 16
 // 0.90 / 0.70, 32 x 32 1.27 / 1.05, 40 x 40 1.41 / 1.42; volumes of 16^3 1.31 / 1.20,
 // of 24^3 with 64 histograms 4.7 / 5.4.
 template <typename T>
 bool band_pays(const wdl_ctx* ctx) {
-  if (ctx->ndim == 2)
-    return ctx->N > (sizeof(T) == 4 ? 48 * 48 : 32 * 32) || std::max(ctx->W, ctx->H) > 64;
+  if (ctx->ndim == 2) {
+    if (std::max(ctx->W, ctx->H) > 64) return true;
+    if (ctx->N <= (sizeof(T) == 4 ? 48 * 48 : 32 * 32)) return false;
+    return sizeof(T) == 8 || !covers_lines<T>(ctx);
+  }
   // volumes: where the sums take a line's every tap
   return std::max({ctx->W, ctx->H, ctx->D}) > (sizeof(T) == 4 ? 48 : 16) || !covers_lines<T>(ctx);
 }
