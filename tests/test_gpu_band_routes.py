@@ -12,13 +12,16 @@ from conftest import rel, rel_scaled
 pytestmark = pytest.mark.gpu
 
 # (W, H, D, K, gamma, fused for FP32, for FP64)
-CASES = [(16, 16, 1, 3, 2.0, False, False), (17, 16, 1, 3, 2.0, False, True), (31, 33, 1, 3, 2.0, False, True),
-         (32, 32, 1, 3, 2.0, True, True), (64, 20, 1, 24, 2.0, True, True), (64, 20, 1, 25, 2.0, False, False),
-         (64, 20, 1, 12, 50.0, True, True), (64, 20, 1, 13, 50.0, False, False), (65, 4, 1, 25, 2.0, True, True),
+CASES = [(16, 16, 1, 3, 2.0, False, True), (8, 16, 1, 4, 2.0, False, True), (8, 16, 1, 5, 2.0, False, False),
+         (17, 16, 1, 9, 2.0, False, True), (31, 33, 1, 3, 2.0, False, True),
+         (32, 32, 1, 3, 2.0, True, True), (32, 32, 1, 32, 2.0, True, True), (64, 20, 1, 24, 2.0, True, True),
+         (64, 20, 1, 25, 2.0, False, False), (64, 20, 1, 12, 50.0, True, True), (64, 20, 1, 13, 50.0, True, False),
+         (64, 20, 1, 16, 50.0, True, False), (64, 20, 1, 17, 50.0, False, False), (65, 4, 1, 25, 2.0, True, True),
          (128, 5, 1, 24, 2.0, False, False), (128, 5, 1, 16, 2.0, True, True), (100, 9, 1, 33, 2.0, False, False),
          (8, 8, 8, 2, 2.0, False, False), (16, 9, 8, 4, 2.0, False, True), (16, 16, 16, 3, 2.0, False, True),
          (17, 16, 16, 3, 2.0, True, True), (40, 11, 10, 16, 2.0, True, True), (40, 11, 10, 17, 2.0, False, False),
-         (40, 33, 7, 10, 60.0, False, False), (32, 13, 11, 20, 60.0, True, True)]
+         (40, 33, 7, 12, 60.0, True, True), (40, 33, 7, 13, 60.0, False, False), (32, 13, 11, 20, 60.0, True, True),
+         (32, 13, 11, 21, 60.0, True, False), (32, 13, 11, 25, 60.0, False, False)]
 
 
 @pytest.mark.parametrize("precision", ["fp32", "fp64"])

@@ -932,9 +932,11 @@ bool band_fits(const wdl_ctx* ctx, int K) {
 // Banded rows / separate kernels / before the banded kernels, ms an evaluation, L = 6 or 8:
 //   atoms x groups of eight: 8 of 64 x 64, K = 64, FP64 4.1 / 2.6 / 3.0; 8 of 32^3, K = 64
 //     33.6 / 19.4 / 23.9; gamma 50, FP64: 64 of 64 x 64 K = 12 2.71 / 2.80 / 2.81, K = 16 3.85 /
-//     3.57 / 3.58; 8 of 40^3 K = 8 4.40 / 4.98 / 5.10, K = 20 15.5 / 12.4 / 11.8
+//     3.57 / 3.58, FP32 K = 16 2.01 / 2.00 / 2.17, K = 20 2.64 / 2.54 / 2.62; 8 of 40^3
+//     K = 8 4.40 / 4.98 / 5.10, K = 20 15.5 / 12.4 / 11.8
 //   pixels: one histogram, K = 5, FP32 16 x 16 0.39 / 0.25 / 0.27, 32 x 32 0.30 / 0.31 / 0.41;
-//     barycenters of 16^3, K = 8, L = 20 0.56 / 0.48 / 0.48
+//     barycenters of 16^3, K = 8, L = 20 0.56 / 0.48 / 0.48; FP64 16 x 16 against before: 1.27 x the speed
+//     with 3 atoms, 1.00 with 8, 0.89 with 16 (2.5 x for 64 histograms)
 //   shared memory, one block on an SM: 24 of 128 x 128, K = 24, FP64 8.6 / 5.3 / 11.7, at gamma
 //     50 12.0 / 7.9 / 11.7; few atoms on long lines want it: 2048 x 64, K = 2 0.46 / 0.68 / 6.3
 template <typename T>
@@ -942,10 +944,15 @@ bool band_rows_pay(const wdl_ctx* ctx, int K) {
   const RowsShape<T> sh(ctx, K);
   const bool vol = ctx->ndim == 3;
   if (std::max({ctx->W, ctx->H, ctx->D}) > 64) return K <= 16 || sh.bwd_smem(K) <= 110 * 1024;
-  if (ctx->N < (sizeof(T) == 4 ? (vol ? 4097 : 1024) : vol ? 513 : 257)) return false;
+  if (ctx->N < (sizeof(T) == 4 ? (vol ? 4097 : 1024) : vol ? 513 : 257) &&
+      (sizeof(T) == 4 || vol || K > (int)(ctx->N / 32)))
+    return false;
   const int items = K * sh.ax.G;
   if (!covers_lines<T>(ctx)) return items <= (vol ? 80 : 192);
-  return items <= (!vol ? 96 : sh.ax.G <= 4 ? 80 : 48);
+  // eight of 32^3, K = 24, gamma 50, FP32: 1.06 x the speed before; of 36^3, K = 14: 0.88 x
+  const bool brief = sh.ax.G <= 4;
+  if (vol) return items <= (!brief ? 64 : sizeof(T) == 4 ? 96 : 80);
+  return items <= (sizeof(T) == 4 || brief ? 128 : 96);
 }
 template bool band_rows_pay<float>(const wdl_ctx*, int);
 template bool band_rows_pay<double>(const wdl_ctx*, int);
